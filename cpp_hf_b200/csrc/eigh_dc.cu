@@ -1,0 +1,598 @@
+// Batched Hermitian eigendecomposition for any nb <= kMaxEighNb (replaces
+// Eigen's SelfAdjointEigenSolver in cpp_hf linalg.hpp:39-120): Householder
+// reduction to a real symmetric tridiagonal, divide and conquer on it, and the
+// back-transformation, one CTA per matrix in one launch.
+//
+// Thread (j, q) = (tid / 4, tid % 4) holds the rows i = 4 ii + q of column j in
+// registers, for the matrix during the reduction and for the eigenvectors
+// during the back-transformation, so both run on register operands with u and
+// p broadcast from shared memory.
+//  1. Reduction, k = 0 .. n-3: H = I - beta u u^H maps A[k+1:, k] to alpha e1;
+//     with p = beta A u, K = beta/2 u^H p and w = p - K u the similarity is the
+//     rank-2 update A -= u w^H + w u^H.  Two block barriers a step.  A unitary
+//     diagonal makes the subdiagonal e real and non-negative.
+//  2. Divide and conquer (Cuppen 1981; Gu and Eisenstat 1995): T is torn at
+//     every off-diagonal, T = diag(d_i - e_{i-1} - e_i) + sum e_i v_i v_i^T, and
+//     neighbouring blocks are merged pairwise, all merges of a level at once.
+//     A merge diagonalises D + rho z z^T: small z and close D deflate; each
+//     other eigenvalue is a root of 1 + rho sum z_i^2 / (d_i - x), found by four
+//     lanes as an offset from its nearest pole by the two-pole rational
+//     iteration (Li 1993) inside a bisection bracket; z is recomputed from the
+//     roots (Loewner's formula), which makes the eigenvectors orthogonal to
+//     rounding; the vectors are the product of the old ones with
+//     z_i / (d_i - x).  No step is a chain longer than one row of the matrix,
+//     unlike the n^2 dependent rotations of QL.
+//  3. The reflectors are applied to the eigenvectors, stored by ascending
+//     eigenvalue (stable) or, with block sizes, block by block.
+// What bounds it: the latency of the n reduction steps (two barriers, a square
+// root and a division each; half of the kernel at nb = 64), then the secular
+// iterations.  Measured against the cyclic Jacobi kernel it replaces (Hermitian
+// matrices with normal entries): 5184 of nb = 64 6.46 ms (84.7), 5184 of nb = 48
+// 3.31 (25.6), 2304 of nb = 32 0.47 (3.28), 9216 of nb = 24 1.07 (7.6), of
+// nb = 16 0.44 (1.29), of nb = 10 0.36 (0.48), 1296 of nb = 80 4.36 (39.2).
+#include "common.cuh"
+#include "eigh.cuh"
+
+#include <mutex>
+
+namespace cpphf {
+
+namespace {
+
+constexpr double kEps = 2.220446049250313e-16;
+constexpr int kSecularMaxIter = 60;  // safeguarded: a bisection of the bracket at worst
+
+template <int NE>
+struct DcGeo {
+    static constexpr int NR = 4 * NE;                     // rows, rounded up
+    static constexpr int NT = 4 * ((NR + 7) / 8 * 8);     // threads: four per column, whole warps
+    static constexpr int LD = NR + 1;                     // row stride of Q and S
+    // CTAs per SM the registers are limited for (the shared memory allows as many)
+    static constexpr int BLOCKS = NE <= 4 ? 12 : NE <= 6 ? 8 : NE <= 8 ? 6 : NE <= 12 ? 3 : NE <= 16 ? 2 : 1;
+};
+
+// Shared memory of one matrix.  U holds the reflectors packed by column.
+template <int NE>
+struct DcSmem {
+    static constexpr int NR = DcGeo<NE>::NR, LD = DcGeo<NE>::LD;
+    double2 U[NR * (NR - 1) / 2];
+    double2 ub[2][NR], pb[2][NR], sub[NR];
+    double Q[NR * LD], S[NR * LD];
+    double beta[NR], d[NR], e[NR], z[NR], ds[NR], zs[NR], dk[NR], zk[NR], mu[NR], zh[NR], rc[NR], rs[NR];
+    double red[2][DcGeo<NE>::NT / 32];
+    int perm[NR], nd[NR], df[NR], org[NR], ra[NR], rb[NR], nrot[NR];
+};
+
+__device__ __forceinline__ double quad_sum(double v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    return v;
+}
+__device__ __forceinline__ int quad_sum(int v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    return v;
+}
+__device__ __forceinline__ double quad_max(double v) {
+    v = fmax(v, __shfl_xor_sync(0xffffffffu, v, 1));
+    return fmax(v, __shfl_xor_sync(0xffffffffu, v, 2));
+}
+
+// Root r of 1 + rho sum_i z_i^2 / (d_i - x), d ascending, as (pole, offset).
+// Called by the four lanes of a quad (q = 0..3 each sum every fourth term; the
+// xor sums leave the same bits in all four) with `on` false for quads without a
+// root, which only take part in the shuffles.
+__device__ __forceinline__ void secular_root(const double* d, const double* z, double rho, int r, int k, int q, bool on,
+                                             int& org, double& mu) {
+    double a = 0.0, b = 0.0;
+    org = r;
+    mu = 0.0;
+    const bool last = r == k - 1;
+    {
+        // the half of the interval with the root: sign of f at its middle
+        const double mid = (on && !last) ? 0.5 * (d[r + 1] - d[r]) : 0.0;
+        double s = 0.0;
+        if (on)
+            for (int i = q; i < k; i += 4) s += last ? z[i] * z[i] : z[i] * z[i] / ((d[i] - d[r]) - mid);
+        s = quad_sum(s);
+        if (on) {
+            if (last) {
+                b = rho * s;
+                mu = b;
+            } else if (1.0 + rho * s >= 0.0) {
+                b = mid;
+                mu = mid;
+            } else {
+                org = r + 1;
+                a = -mid;
+                mu = -mid;
+            }
+        }
+    }
+    const double dorg = on ? d[org] : 0.0;
+    bool run = on;
+    for (int it = 0; it < kSecularMaxIter; ++it) {
+        if (!__any_sync(0xffffffffu, run)) break;
+        double psi = 0.0, dpsi = 0.0, phi = 0.0, dphi = 0.0;
+        if (run) {
+            for (int i = q; i < k; i += 4) {
+                const double t = 1.0 / ((d[i] - dorg) - mu);
+                const double v = rho * z[i] * z[i] * t, dv = v * t;
+                if (i <= r) {
+                    psi += v;
+                    dpsi += dv;
+                } else {
+                    phi += v;
+                    dphi += dv;
+                }
+            }
+        }
+        psi = quad_sum(psi);
+        dpsi = quad_sum(dpsi);
+        phi = quad_sum(phi);
+        dphi = quad_sum(dphi);
+        if (!run) continue;
+        const double w = 1.0 + psi + phi;
+        if (!(fabs(w) > kEps * k * (1.0 + fabs(psi) + fabs(phi)))) {
+            run = false;
+            continue;
+        }
+        if (w < 0.0)
+            a = mu;
+        else
+            b = mu;
+        const double d1 = (d[r] - dorg) - mu;
+        double eta;
+        if (!last) {
+            const double d2 = (d[r + 1] - dorg) - mu;
+            const double c = w - d1 * dpsi - d2 * dphi;
+            const double A = (d1 + d2) * w - d1 * d2 * (dpsi + dphi), B = d1 * d2 * w;
+            const double disc = sqrt(fabs(A * A - 4.0 * B * c));
+            eta = c == 0.0 ? B / A : (A <= 0.0 ? (A - disc) / (2.0 * c) : 2.0 * B / (A + disc));
+        } else {
+            eta = d1 + d1 * d1 * dpsi / (w - d1 * dpsi);
+        }
+        if (!(w * eta < 0.0)) eta = -w / (dpsi + dphi);
+        double next = mu + eta;
+        if (!(next > a && next < b)) next = 0.5 * (a + b);
+        if (next == mu)
+            run = false;
+        else
+            mu = next;
+    }
+}
+
+// Input transform: mode 0 -> herm(M), 1 -> herm(i M).
+template <int NE>
+__global__ void __launch_bounds__(DcGeo<NE>::NT, DcGeo<NE>::BLOCKS)
+    k_eigh_dc(const double2* __restrict__ M, double* __restrict__ w, double2* __restrict__ Vout, int n, int mode,
+              const BlockSpec bs) {
+    constexpr int LD = DcGeo<NE>::LD, NR = DcGeo<NE>::NR, NW = DcGeo<NE>::NT / 32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    DcSmem<NE>& s = *reinterpret_cast<DcSmem<NE>*>(smem_raw);
+    const int tid = threadIdx.x, q = tid & 3, j = tid >> 2, warp = tid >> 5, lane = tid & 31;
+    const double2* Mk = M + (size_t)blockIdx.x * n * n;
+    double* wk = w + (size_t)blockIdx.x * n;
+    double2* Vk = Vout + (size_t)blockIdx.x * n * n;
+
+    // ---- load, hermitise, scale by a power of two (exact) to O(1) ----
+    double2 a[NE];
+    double amax = 0.0;
+    bool bad = false;
+#pragma unroll
+    for (int ii = 0; ii < NE; ++ii) {
+        const int i = 4 * ii + q;
+        double2 h = mk(0.0, 0.0);
+        if (i < n && j < n && !(bs.nblocks > 1 && bs.blk[i] != bs.blk[j])) {
+            double2 x = Mk[i * n + j], y = Mk[j * n + i];
+            if (mode == 1) {
+                x = mk(-x.y, x.x);
+                y = mk(-y.y, y.x);
+            }
+            h = mk(0.5 * (x.x + y.x), i == j ? 0.0 : 0.5 * (x.y - y.y));
+            bad = bad || !isfinite(h.x) || !isfinite(h.y);
+            amax = fmax(amax, fmax(fabs(h.x), fabs(h.y)));
+        }
+        a[ii] = h;
+    }
+    amax = warp_max(amax);
+    if (lane == 0) s.red[0][warp] = amax;
+    if (__syncthreads_or(bad)) {  // a NaN or infinity: no decomposition
+        for (int t = tid; t < n * n; t += blockDim.x) Vk[t] = mk((double)NAN, (double)NAN);
+        for (int t = tid; t < n; t += blockDim.x) wk[t] = NAN;
+        return;
+    }
+    for (int t = 0; t < NW; ++t) amax = fmax(amax, s.red[0][t]);
+    int ex = 0;
+    if (amax > 0.0) frexp(amax, &ex);
+#pragma unroll
+    for (int ii = 0; ii < NE; ++ii) a[ii] = mk(ldexp(a[ii].x, -ex), ldexp(a[ii].y, -ex));
+    __syncthreads();
+
+    // ---- 1. reduction ----
+    for (int k = 0; k + 2 < n; ++k) {
+        const int b = k & 1;
+        double2* u = s.ub[b];
+        double2* p = s.pb[b];
+        if (j == k) {
+            const unsigned quad = 0xfu << (lane & 28);
+            double xn2 = 0.0;
+            double2 x0 = mk(0.0, 0.0);
+#pragma unroll
+            for (int ii = 0; ii < NE; ++ii) {
+                const int i = 4 * ii + q;
+                if (i > k) xn2 += a[ii].x * a[ii].x + a[ii].y * a[ii].y;
+                if (i == k + 1) x0 = a[ii];
+                if (i == k) s.d[k] = a[ii].x;
+            }
+            xn2 += __shfl_xor_sync(quad, xn2, 1);
+            xn2 += __shfl_xor_sync(quad, xn2, 2);
+            const int src = (lane & 28) + ((k + 1) & 3);
+            x0 = mk(__shfl_sync(quad, x0.x, src), __shfl_sync(quad, x0.y, src));
+            const double ax0 = sqrt(fma(x0.x, x0.x, x0.y * x0.y)), xn = sqrt(xn2);
+            const double2 ph = ax0 > 0.0 ? mk(x0.x / ax0, x0.y / ax0) : mk(1.0, 0.0);
+            double2* Uk = s.U + (size_t)k * (n - 1) - (size_t)k * (k - 1) / 2 - (k + 1);
+#pragma unroll
+            for (int ii = 0; ii < NE; ++ii) {
+                const int i = 4 * ii + q;
+                if (i > k && i < n) {
+                    const double2 ui = i == k + 1 ? mk(x0.x + ph.x * xn, x0.y + ph.y * xn) : a[ii];
+                    u[i] = ui;
+                    Uk[i] = ui;
+                }
+            }
+            if (q == 0) {
+                s.beta[k] = xn > 0.0 ? 1.0 / (xn * (xn + ax0)) : 0.0;
+                s.sub[k] = xn > 0.0 ? mk(-ph.x * xn, -ph.y * xn) : x0;
+            }
+        }
+        __syncthreads();
+        const double beta = s.beta[k];
+        const bool on = beta != 0.0 && j > k && j < n;
+        double2 pj = mk(0.0, 0.0), uj = mk(0.0, 0.0);
+        const int ii0 = (k + 1) >> 2;
+        if (warp * 8 + 7 > k) {  // the warp holds an active column
+            double2 p0 = mk(0.0, 0.0), p1 = mk(0.0, 0.0);
+            if (on) {
+#pragma unroll
+                for (int ii = 0; ii < NE; ++ii) {
+                    const int i = 4 * ii + q;
+                    if (ii >= ii0 && i > k && i < n) cfma((ii & 1) ? p1 : p0, cconj(a[ii]), u[i]);
+                }
+                uj = u[j];
+            }
+            pj = mk(quad_sum(p0.x + p1.x) * beta, quad_sum(p0.y + p1.y) * beta);
+            double kp = (q == 0) ? uj.x * pj.x + uj.y * pj.y : 0.0;
+            kp = warp_sum(kp);
+            if (lane == 0) s.red[b][warp] = kp;
+            if (on && q == 0) p[j] = pj;
+        } else if (lane == 0) {
+            s.red[b][warp] = 0.0;
+        }
+        __syncthreads();
+        if (on) {
+            double kp = 0.0;
+#pragma unroll
+            for (int t = 0; t < NW; ++t) kp += s.red[b][t];
+            const double K = 0.5 * beta * kp;
+            const double2 cw = mk(pj.x - K * uj.x, -(pj.y - K * uj.y)), cu = cconj(uj);
+#pragma unroll
+            for (int ii = 0; ii < NE; ++ii) {
+                const int i = 4 * ii + q;
+                if (ii >= ii0 && i > k && i < n) {
+                    const double2 ui = u[i], pi = p[i];
+                    const double2 wi = mk(pi.x - K * ui.x, pi.y - K * ui.y);
+                    a[ii] = csub(a[ii], cmul(ui, cw));
+                    a[ii] = csub(a[ii], cmul(wi, cu));
+                }
+            }
+        }
+    }
+    // the last two diagonal entries and the last subdiagonal
+#pragma unroll
+    for (int ii = 0; ii < NE; ++ii) {
+        const int i = 4 * ii + q;
+        if (j < n && j + 2 >= n && i == j) s.d[j] = a[ii].x;
+        if (j + 2 == n && i == j + 1) s.sub[j] = a[ii];
+    }
+    for (int t = tid; t < NR * LD; t += blockDim.x) s.Q[t] = (t % LD == t / LD) ? 1.0 : 0.0;
+    __syncthreads();
+
+    // ---- real tridiagonal: e_i = |sub_i|, delta_{i+1} = delta_i sub_i / |sub_i| ----
+    double2* delta = s.ub[0];
+    if (q == 0 && j < n) {
+        double ej = 0.0;
+        if (j + 1 < n) ej = sqrt(fma(s.sub[j].x, s.sub[j].x, s.sub[j].y * s.sub[j].y));
+        s.e[j] = ej;
+        double2 x = mk(1.0, 0.0);
+        if (j > 0) {
+            const double2 v = s.sub[j - 1];
+            const double m = sqrt(fma(v.x, v.x, v.y * v.y));
+            if (m > 0.0) x = mk(v.x / m, v.y / m);
+        }
+        delta[j] = x;
+    }
+    __syncthreads();
+    for (int st = 1; st < n; st *= 2) {  // inclusive product
+        double2 x = mk(1.0, 0.0);
+        const bool act = q == 0 && j < n && j >= st;
+        if (act) x = cmul(delta[j], delta[j - st]);
+        __syncthreads();
+        if (act) delta[j] = x;
+        __syncthreads();
+    }
+    if (q == 0 && j < n) {
+        const double2 x = delta[j];
+        const double m = 1.0 / sqrt(fma(x.x, x.x, x.y * x.y));
+        delta[j] = mk(x.x * m, x.y * m);
+        s.d[j] = s.d[j] - (j > 0 ? s.e[j - 1] : 0.0) - s.e[j];
+    }
+    __syncthreads();
+
+    // ---- 2. divide and conquer ----
+    for (int half = 1; half < n; half *= 2) {
+        const int lo = j / (2 * half) * (2 * half), mid = min(lo + half, n), hi = min(lo + 2 * half, n);
+        const bool on = j < n && mid < hi;  // this column's block is merged at this level
+        const int len = on ? hi - lo : 0;
+        const double rho = on ? 2.0 * s.e[mid - 1] : 0.0;
+        const double zj = on ? 0.70710678118654752440 * s.Q[(j < mid ? mid - 1 : mid) * LD + j] : 0.0;
+        const double dj = on ? s.d[j] : 0.0;
+        if (on && q == 0) s.z[j] = zj;
+        __syncthreads();
+        int rank = 0;
+        double dmax = 0.0, zmax = 0.0;
+        for (int i = lo + q; i < lo + len; i += 4) {
+            const double di = s.d[i];
+            rank += (di < dj || (di == dj && i < j)) ? 1 : 0;
+            dmax = fmax(dmax, fabs(di));
+            zmax = fmax(zmax, fabs(s.z[i]));
+        }
+        rank = quad_sum(rank);
+        const double tol = 8.0 * kEps * fmax(quad_max(dmax), quad_max(zmax));
+        if (on && q == 0) {
+            const int at = lo + rank;
+            s.ds[at] = dj;
+            s.zs[at] = zj;
+            s.perm[at] = j;
+            s.df[at] = rho * fabs(zj) <= tol;
+        }
+        if (on && q == 1) s.nrot[j] = 0;
+        __syncthreads();
+        // from here on j is a position in the sorted order of its block
+        bool close = false;
+        if (on && q == 0 && !s.df[j]) {
+            int pv = j - 1;
+            while (pv >= lo && s.df[pv]) --pv;
+            if (pv >= lo) {
+                const double x = s.zs[pv], c = s.zs[j];
+                close = fabs((s.ds[j] - s.ds[pv]) * x * c) <= tol * (x * x + c * c);
+            }
+        }
+        if (__syncthreads_or(close)) {
+            // rotate each close pair so that one of its z vanishes (in order: a
+            // rotated entry may be close to the next one)
+            if (on && q == 0 && j == lo) {
+                int pv = -1, nr = 0;
+                for (int i = lo; i < hi; ++i) {
+                    if (s.df[i]) continue;
+                    if (pv >= 0) {
+                        double x = s.zs[pv], c = s.zs[i];
+                        const double dp = s.ds[pv], di = s.ds[i];
+                        if (fabs((di - dp) * x * c) <= tol * (x * x + c * c)) {
+                            const double tau = hypot(c, x);
+                            c /= tau;
+                            x = -x / tau;
+                            s.zs[i] = tau;
+                            s.zs[pv] = 0.0;
+                            s.ds[pv] = dp * c * c + di * x * x;
+                            s.ds[i] = dp * x * x + di * c * c;
+                            s.df[pv] = 1;
+                            s.ra[lo + nr] = s.perm[pv];
+                            s.rb[lo + nr] = s.perm[i];
+                            s.rc[lo + nr] = c;
+                            s.rs[lo + nr] = x;
+                            ++nr;
+                        }
+                    }
+                    pv = i;
+                }
+                s.nrot[lo] = nr;
+            }
+            __syncthreads();
+            if (on && q == 0) {  // row j of the block
+                const int nr = s.nrot[lo];
+                for (int t = 0; t < nr; ++t) {
+                    const int ca = s.ra[lo + t], cb = s.rb[lo + t];
+                    const double c = s.rc[lo + t], x = s.rs[lo + t];
+                    const double va = s.Q[j * LD + ca], vb = s.Q[j * LD + cb];
+                    s.Q[j * LD + ca] = c * va + x * vb;
+                    s.Q[j * LD + cb] = c * vb - x * va;
+                }
+            }
+            __syncthreads();
+        }
+        // positions of the k undeflated entries first, then the deflated ones
+        int k = 0, before = 0;
+        for (int i = lo + q; i < lo + len; i += 4) {
+            const int live = s.df[i] ? 0 : 1;
+            k += live;
+            before += i < j ? live : 0;
+        }
+        k = quad_sum(k);
+        before = quad_sum(before);
+        if (on && q == 0) {
+            const bool live = !s.df[j];
+            const int at = live ? lo + before : lo + k + (j - lo - before);
+            s.nd[at] = j;
+            if (live) {
+                s.dk[at] = s.ds[j];
+                s.zk[at] = s.zs[j];
+            }
+        }
+        __syncthreads();
+        const int r = j - lo;
+        const bool root = on && r < k;
+        int org;
+        double mu;
+        secular_root(s.dk + lo, s.zk + lo, rho, r, k, q, root, org, mu);
+        if (root && q == 0) {
+            s.org[j] = org;
+            s.mu[j] = mu;
+        }
+        __syncthreads();
+        // z from the computed roots: z_i^2 = prod_t (x_t - d_i) / prod_{t != i} (d_t - d_i)
+        {
+            double pr = 1.0;
+            if (root) {
+                const double di = s.dk[j];
+                for (int t = q; t < k; t += 4) {
+                    const double num = (s.dk[lo + s.org[lo + t]] - di) + s.mu[lo + t];
+                    pr *= t == r ? num : num / (s.dk[lo + t] - di);
+                }
+            }
+            pr *= __shfl_xor_sync(0xffffffffu, pr, 1);
+            pr *= __shfl_xor_sync(0xffffffffu, pr, 2);
+            if (root && q == 0) s.zh[j] = copysign(sqrt(fabs(pr)), s.zk[j]);
+        }
+        __syncthreads();
+        double dnew = 0.0;
+        {
+            double nrm = 0.0;
+            if (root) {
+                const double dorg = s.dk[lo + org];
+                dnew = dorg + mu;
+                for (int t = q; t < k; t += 4) {
+                    const double v = s.zh[lo + t] / ((s.dk[lo + t] - dorg) - mu);
+                    s.S[t * LD + j] = v;
+                    nrm += v * v;
+                }
+            }
+            nrm = quad_sum(nrm);
+            const double inv = nrm > 0.0 ? 1.0 / sqrt(nrm) : 0.0;
+            if (root)
+                for (int t = q; t < k; t += 4) s.S[t * LD + j] *= inv;
+        }
+        __syncwarp();
+        double acc[NE];
+#pragma unroll
+        for (int ii = 0; ii < NE; ++ii) acc[ii] = 0.0;
+        if (root) {
+            const bool mixed = s.nrot[lo] > 0;  // a rotation joined columns of both halves
+            for (int t = 0; t < k; ++t) {
+                const int c = s.perm[s.nd[lo + t]];
+                const double v = s.S[t * LD + j];
+                const double* Qc = s.Q + q * LD + c;
+                // without rotations column c is zero outside its half
+                const int i0 = (c < mid || mixed ? lo : mid) >> 2, i1 = ((c >= mid || mixed ? hi : mid) + 3) >> 2;
+#pragma unroll
+                for (int ii = 0; ii < NE; ++ii)
+                    if (ii >= i0 && ii < i1) acc[ii] = fma(Qc[4 * ii * LD], v, acc[ii]);
+            }
+        } else if (on) {
+            const int at = s.nd[j], c = s.perm[at];
+            dnew = s.ds[at];
+#pragma unroll
+            for (int ii = 0; ii < NE; ++ii) acc[ii] = s.Q[(4 * ii + q) * LD + c];
+        }
+        __syncthreads();
+        if (on) {
+            if (q == 0) s.d[j] = dnew;
+#pragma unroll
+            for (int ii = 0; ii < NE; ++ii) {
+                const int i = 4 * ii + q;
+                if (i >= lo && i < hi) s.Q[i * LD + j] = acc[ii];
+            }
+        }
+        __syncthreads();
+    }
+
+    // ---- 3. order, back-transformation ----
+    const double dj = j < n ? s.d[j] : 0.0;
+    int rank = 0;
+    if (bs.nblocks > 1 && !bs.sort) {
+        // the vectors of a block-diagonal matrix keep to one block each: the block
+        // of a vector is that of its largest entry
+        if (j < n && q == 0) {
+            int im = 0;
+            double vm = -1.0;
+            for (int i = 0; i < n; ++i)
+                if (fabs(s.Q[i * LD + j]) > vm) {
+                    vm = fabs(s.Q[i * LD + j]);
+                    im = i;
+                }
+            s.nd[j] = bs.blk[im];
+        }
+        __syncthreads();
+        if (j < n)
+            for (int i = q; i < n; i += 4) {
+                const double di = s.d[i];
+                const int bi = s.nd[i], bj = s.nd[j];
+                rank += (bi < bj || (bi == bj && (di < dj || (di == dj && i < j)))) ? 1 : 0;
+            }
+    } else if (j < n) {
+        for (int i = q; i < n; i += 4) {
+            const double di = s.d[i];
+            rank += (di < dj || (di == dj && i < j)) ? 1 : 0;
+        }
+    }
+    rank = quad_sum(rank);
+#pragma unroll
+    for (int ii = 0; ii < NE; ++ii) {
+        const int i = 4 * ii + q;
+        a[ii] = mk(0.0, 0.0);
+        if (i < n && j < n) a[ii] = cscale(delta[i], s.Q[i * LD + j]);
+    }
+    for (int k = n - 3; k >= 0; --k) {
+        const double beta = s.beta[k];
+        if (beta == 0.0) continue;
+        const double2* Uk = s.U + (size_t)k * (n - 1) - (size_t)k * (k - 1) / 2 - (k + 1);
+        const int ii0 = (k + 1) >> 2;
+        double2 t0 = mk(0.0, 0.0), t1 = mk(0.0, 0.0);
+#pragma unroll
+        for (int ii = 0; ii < NE; ++ii) {
+            const int i = 4 * ii + q;
+            if (ii >= ii0 && i > k && i < n) cfma((ii & 1) ? t1 : t0, cconj(Uk[i]), a[ii]);
+        }
+        const double2 t = mk(beta * quad_sum(t0.x + t1.x), beta * quad_sum(t0.y + t1.y));
+#pragma unroll
+        for (int ii = 0; ii < NE; ++ii) {
+            const int i = 4 * ii + q;
+            if (ii >= ii0 && i > k && i < n) a[ii] = csub(a[ii], cmul(Uk[i], t));
+        }
+    }
+    if (j < n) {
+        if (q == 0) wk[rank] = ldexp(dj, ex);
+#pragma unroll
+        for (int ii = 0; ii < NE; ++ii) {
+            const int i = 4 * ii + q;
+            if (i < n) Vk[(size_t)i * n + rank] = a[ii];
+        }
+    }
+}
+
+template <int NE>
+int launch(const double2* M, double* w, double2* V, int64_t batch, int nb, int mode, const BlockSpec& bs,
+           cudaStream_t st) {
+    static std::once_flag once;
+    std::call_once(once, [] { raise_smem(k_eigh_dc<NE>); });
+    k_eigh_dc<NE><<<(unsigned)batch, DcGeo<NE>::NT, sizeof(DcSmem<NE>), st>>>(M, w, V, nb, mode, bs);
+    CPPHF_LAUNCH_CHECK("eigh (divide and conquer)");
+    return CPPHF_OK;
+}
+
+}  // namespace
+
+int eigh_dc(const double2* M, double* w, double2* V, int64_t batch, int64_t nb, int mode, const BlockSpec& bs,
+            cudaStream_t st) {
+    static_assert(kMaxEighNb <= 80, "largest size class");
+    // size classes: a thread holds ceil(nb / 4) rows of its column
+    const int n = (int)nb;
+    if (n <= 16) return launch<4>(M, w, V, batch, n, mode, bs, st);
+    if (n <= 24) return launch<6>(M, w, V, batch, n, mode, bs, st);
+    if (n <= 32) return launch<8>(M, w, V, batch, n, mode, bs, st);
+    if (n <= 48) return launch<12>(M, w, V, batch, n, mode, bs, st);
+    if (n <= 64) return launch<16>(M, w, V, batch, n, mode, bs, st);
+    return launch<20>(M, w, V, batch, n, mode, bs, st);
+}
+
+}  // namespace cpphf
