@@ -38,6 +38,9 @@ __device__ __forceinline__ double2 scf_mix_herm(double2 mij, double2 mji) {
 
 int dm_check_nb(int64_t nb);
 int dm_density(const double2* Q, const double* p, double2* P, int64_t nk, int nb, cudaStream_t st);
+// density with the occupations p = expit((mu - e) / T) formed in the same pass
+int dm_dens_occ(const double2* Q, const double* e, const double* mu, double T, double* p, double2* P, int64_t nk, int nb,
+                cudaStream_t st);
 int dm_rotate(const double2* U, const double2* M, double2* Out, double* eps, int64_t nk, int nb, cudaStream_t st);
 int dm_q_times_u(double2* Q, const double2* U, int64_t nk, int nb, cudaStream_t st);
 int dm_occupations(const double* eps, const double* mu, double T_r, double* p, int64_t n, cudaStream_t st);
@@ -49,14 +52,5 @@ int dm_pr_beta(const double2* G, const double2* Gp, const double* g_p, const dou
 int dm_direction(const double2* G, const double2* dQp, const double* g_p, const double* dpp, const double* eps,
                  const double* p, const double* w, double2* dQ, double* d_p, int64_t nk, int nb, double T_r,
                  double max_step, DmScalars* S, cudaStream_t st);
-int dm_trial(const double2* V, const double2* Fe, const double* lam, const double* p, const double* d_p,
-             const double* w, int64_t nk, int nb, double T_r, double shrink, int last_trial, double fallback,
-             DmScalars* S, cudaStream_t st);
-int dm_trial_lu(const double2* dQ, const double2* Ft, const double* p, const double* d_p, const double* w, int64_t nk,
-                int nb, double T_r, double shrink, int last_trial, double fallback, DmScalars* S, cudaStream_t st);
-int dm_retract_lu(double2* Q, const double2* dQ, const double2* Ft, double* ew, int64_t nk, int nb, const DmScalars* S,
-                  cudaStream_t st);
-int dm_retract(double2* Q, const double2* V, const double2* Fe, const double* lam, double* ew, int64_t nk, int nb,
-               const DmScalars* S, cudaStream_t st);
 
 }  // namespace cpphf

@@ -1,5 +1,5 @@
 // Direct-minimisation per-k kernels specialised for small band counts
-// (nb in {2, 4, 6, 8}; cpp_hf solver_dm.hpp:117-344).
+// (2 <= nb <= 8; cpp_hf solver_dm.hpp:117-344).
 //
 // Tile kernels (density, rotation + gradient, Cayley trial, retraction): a
 // group of GS = (nb rounded up to a power of two) threads owns one k-point and
@@ -787,7 +787,7 @@ int resident_ctas(K kern, size_t smem) {
 
 }  // namespace
 
-bool dm_small_supported(int nb) { return nb == 2 || nb == 4 || nb == 6 || nb == 8; }
+bool dm_small_supported(int nb) { return nb >= 2 && nb <= 8; }
 
 int dm_small_dens_occ(const double2* Q, const double* ew, const double* mu, double T_r, double* p, double2* P,
                       int64_t nk, int nb, cudaStream_t st) {

@@ -1,4 +1,4 @@
-// Internal interface of the small-nb (2, 4, 6, 8) direct-minimisation kernels.
+// Internal interface of the small-nb (2 <= nb <= 8) direct-minimisation kernels.
 #pragma once
 
 #include "common.cuh"

@@ -38,7 +38,7 @@ int solve_rtr(const cpphf_kernel* K, const cpphf_dm_config* cfg, const double2* 
               cpphf_project_fn project, void* puser, double2* Q_out, double* p_out, double2* D_out, double2* F_out,
               double* hist_E, double* hist_G, cpphf_dm_result* res, void* ws, size_t wsb, cudaStream_t st);
 
-// Tiled kernels for nb in {2, 4, 6, 8} (rtr_small.cu); same contracts as the
+// Tiled kernels for 2 <= nb <= 8 (rtr_small.cu); same contracts as the
 // team kernels of rtr.cu.  Direction modes: 0 d = z(r), 1 d = z(r) + beta d,
 // 2 d given, 3 as 1 with beta and shift_z formed on the device from the update
 // pass's sums and rz_old.

@@ -1,4 +1,4 @@
-// Trust-region Newton per-k kernels for small band counts (nb in {2, 4, 6, 8};
+// Trust-region Newton per-k kernels for small band counts (2 <= nb <= 8;
 // cpp_hf solver_rtr.hpp:55-111, 380-396).  Same tile scheme as the small-nb
 // direct-minimisation kernels: a group of GS threads owns one k-point, thread r
 // owns row r of every matrix, tiles of KT k-points are staged through shared
@@ -430,7 +430,7 @@ void rtr_small_attrs() {
 
 }  // namespace
 
-bool rtr_small_supported(int nb) { return nb == 2 || nb == 4 || nb == 6 || nb == 8; }
+bool rtr_small_supported(int nb) { return nb >= 2 && nb <= 8; }
 
 int rtr_small_direction(const double2* rX, const double* rp, const double* eps, const double* p, const double* w,
                         const double2* Q, const double2* vX, const double* vp, double2* dX, double* dp, double2* dP,

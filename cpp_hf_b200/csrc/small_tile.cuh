@@ -1,4 +1,4 @@
-// Tile helpers of the small-nb (2, 4, 6, 8) per-k kernels: a group of GS
+// Tile helpers of the small-nb (2 <= nb <= 8) per-k kernels: a group of GS
 // threads (nb rounded up to a power of two) owns one k-point, thread r owns row
 // r of every matrix, and a CTA of kThreads threads stages KT = kThreads / GS
 // k-points per tile through shared memory (coalesced loads and stores into a
@@ -323,8 +323,11 @@ inline unsigned tiles_grid(int64_t nk, int KT, int cap) {
 #define SMALL_DISPATCH(nb, X) \
     switch (nb) {             \
         case 2: X(2); break;  \
+        case 3: X(3); break;  \
         case 4: X(4); break;  \
+        case 5: X(5); break;  \
         case 6: X(6); break;  \
+        case 7: X(7); break;  \
         case 8: X(8); break;  \
         default: return fail(CPPHF_ERR_UNSUPPORTED, "small-nb kernel called with unsupported nb"); \
     }

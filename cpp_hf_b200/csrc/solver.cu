@@ -6,6 +6,7 @@
 // few scalars its convergence test needs.
 #include "common.cuh"
 #include "dm.cuh"
+#include "dm_mma.cuh"
 #include "dm_small.cuh"
 #include "eigh.cuh"
 #include "fock.cuh"
@@ -68,57 +69,6 @@ __global__ void k_level_shift(const double* __restrict__ eps, const double* __re
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double occ = expit_d(-(eps[i] - m) / (T + 1.0e-12));
         shifted[i] = eps[i] + ls * (1.0 - occ);
-    }
-}
-
-__global__ void k_fermi(const double* __restrict__ e, const double* __restrict__ mu, double T, double* __restrict__ occ,
-                        int64_t n) {
-    const double m = *mu;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        occ[i] = expit_d(-(e[i] - m) / (T + 1.0e-12));
-}
-
-// SCF residuals: delta = P_new - D, comm = F D - D F; weighted squared norms.
-// One team per k (solver_scf.hpp:224-242, 64-75).
-template <bool WARP>
-__global__ void k_scf_residuals(const double2* __restrict__ F, const double2* __restrict__ D,
-                                const double2* __restrict__ Pn, const double* __restrict__ w, int64_t nk, int nb,
-                                DmScalars* S, double2* __restrict__ comm_out) {
-    extern __shared__ __align__(16) unsigned char raw[];
-    __shared__ double red[64];
-    Team<WARP> t;
-    const int ld = nb + 1;
-    const size_t per = (sizeof(double2) * team_mat_elems(nb) * 2 + 15) & ~(size_t)15;
-    double2* Fs = reinterpret_cast<double2*>(raw + per * t.team);
-    double2* Ds = Fs + team_mat_elems(nb);
-    double v[2] = {0.0, 0.0};
-    for (int64_t k = (int64_t)blockIdx.x * t.nteams + t.team; k < nk; k += (int64_t)gridDim.x * t.nteams) {
-        tload<WARP>(Fs, F + (size_t)k * nb * nb, nb, t);
-        tload<WARP>(Ds, D + (size_t)k * nb * nb, nb, t);
-        t.sync();
-        const double wk = w[k];
-        double sd = 0.0, sc = 0.0;
-        for (int e = t.tid; e < nb * nb; e += t.nt) {
-            const int i = e / nb, j = e - i * nb;
-            const double2 d = csub(Pn[(size_t)k * nb * nb + e], Ds[i * ld + j]);
-            sd += d.x * d.x + d.y * d.y;
-            double2 fp = mk(0.0, 0.0), pf = mk(0.0, 0.0);
-            for (int l = 0; l < nb; ++l) {
-                cfma(fp, Fs[i * ld + l], Ds[l * ld + j]);
-                cfma(pf, Ds[i * ld + l], Fs[l * ld + j]);
-            }
-            const double2 c = csub(fp, pf);
-            if (comm_out) comm_out[(size_t)k * nb * nb + e] = c;
-            sc += c.x * c.x + c.y * c.y;
-        }
-        v[0] += wk * sd;
-        v[1] += wk * sc;
-        t.sync();
-    }
-    double out[2];
-    if (reduce_last_block<2>(v, S->part, &S->counter, out, red) && threadIdx.x == 0) {
-        S->grad_norm = out[0];  // density residual^2 * weight_sum
-        S->lam_pc = out[1];     // commutator residual^2 * weight_sum
     }
 }
 
@@ -553,14 +503,9 @@ int solve_dm(const cpphf_kernel* K, const cpphf_dm_config* cfg, const double2* P
     }
 
     const bool small = dm_small_supported(nb);
-    // density from (Q, occupations); small nb fuses p = expit((mu - ew)/T_r)
+    // density from (Q, occupations p = expit((mu - ew)/T_r))
     auto density = [&](const double* ewv) -> int {
-        if (small) {
-            CPPHF_TRY(dm_small_dens_occ(Q, ewv, &S->mu, T_r, p, P, nk, nb, st));
-        } else {
-            CPPHF_TRY(dm_occupations(ewv, &S->mu, T_r, p, nk * nb, st));
-            CPPHF_TRY(dm_density(Q, p, P, nk, nb, st));
-        }
+        CPPHF_TRY(dm_dens_occ(Q, ewv, &S->mu, T_r, p, P, nk, nb, st));
         if (project) {
             CPPHF_TRY(call_project(project, puser, P, K, st));
             CPPHF_TRY(hermitize(P, P, nk, nb, st));
@@ -617,8 +562,7 @@ int solve_dm(const cpphf_kernel* K, const cpphf_dm_config* cfg, const double2* P
             CPPHF_TRY(dm_small_direction(G[cur], dQ[prv], g[cur], dp[prv], eps, p, wn, dQ[cur], dp[cur], nk, nb, T_r,
                                          cfg->max_step, S, st));
         } else {
-            CPPHF_TRY(dm_rotate(Q, F, F, eps, nk, nb, st));
-            CPPHF_TRY(dm_gradient(F, p, eps, wn, G[cur], g[cur], nk, nb, T_r, cfg->denom_scale, S, st));
+            CPPHF_TRY(dm_mma_rot_grad(Q, F, p, wn, eps, G[cur], g[cur], nk, nb, T_r, cfg->denom_scale, S, st));
             CPPHF_TRY(dm_pr_beta(G[cur], G[prv], g[cur], g[prv], eps, p, wn, nk, nb, T_r, (int)cfg->cg_restart, S,
                                  st));
             CPPHF_TRY(dm_direction(G[cur], dQ[prv], g[cur], dp[prv], eps, p, wn, dQ[cur], dp[cur], nk, nb, T_r,
@@ -626,7 +570,8 @@ int solve_dm(const cpphf_kernel* K, const cpphf_dm_config* cfg, const double2* P
         }
         // 5. Cayley line search (elimination form of the spectral Cayley factor):
         // small nb, two trials per pass; otherwise one pass per trial; a pass
-        // after the accepted trial returns at once
+        // after the accepted trial returns at once.  The trial leaves its factor U
+        // and eps_work for the retraction.
         if (small) {
             // the factors U go to G[prv] and dQ[prv], which this iteration no
             // longer reads (PR+ and the direction are done; the next iteration
@@ -636,14 +581,14 @@ int solve_dm(const cpphf_kernel* K, const cpphf_dm_config* cfg, const double2* P
                                           cfg->bt_shrink, (int)bt, (int)cfg->bt_max, fallback, S, st));
         } else {
             for (int64_t bt = 0; bt < cfg->bt_max; ++bt)
-                CPPHF_TRY(dm_trial_lu(dQ[cur], F, p, dp[cur], wn, nk, nb, T_r, cfg->bt_shrink,
-                                      bt == cfg->bt_max - 1, fallback, S, st));
+                CPPHF_TRY(dm_mma_trial(dQ[cur], F, p, dp[cur], wn, ew, G[prv], nk, nb, T_r, cfg->bt_shrink,
+                                       bt == cfg->bt_max - 1, fallback, S, st));
         }
         // 6. retraction and mu (occupations are formed by the next density step)
         if (small)
             CPPHF_TRY(dm_small_retract(Q, dQ[cur], F, ew, ew2, G[prv], dQ[prv], nk, nb, S, st));
         else
-            CPPHF_TRY(dm_retract_lu(Q, dQ[cur], F, ew, nk, nb, S, st));
+            CPPHF_TRY(dm_mma_retract(Q, dQ[cur], F, ew, G[prv], nk, nb, S, st));
         CPPHF_TRY(mu_solve(ew, wn, nk, nb, n_t, &S->mu, T_r, mu_it, 1, &S->mu, mws, L.mu_bytes, st));
         return CPPHF_OK;
     };
@@ -888,15 +833,9 @@ int solve_scf(const cpphf_kernel* K, const cpphf_scf_config* cfg, const double2*
             CPPHF_TRY(mu_solve(e_occ, K->w2d, nk, nb, n_e, mu_fin, K->T, 30, 0, mu_fin, mws, L.mu_bytes, st));
         // the density pass writes (X + X^H) / 2, exactly Hermitian: only a projector
         // needs the hermitisation again
-        if (dm_small_supported(nb)) {
-            // occupations expit((mu - e) / (T + 1e-12)) formed inside the density pass:
-            // the same value as k_fermi's expit(-(e - mu) / (T + 1e-12)), one launch less
-            CPPHF_TRY(dm_small_dens_occ(V, e_occ, mu_fin, K->T + 1.0e-12, occ, Pout, nk, nb, st));
-        } else {
-            k_fermi<<<grid_for(nk * nb, 256), 256, 0, st>>>(e_occ, mu_fin, K->T, occ, nk * nb);
-            CPPHF_LAUNCH_CHECK("fermi");
-            CPPHF_TRY(dm_density(V, occ, Pout, nk, nb, st));
-        }
+        // occupations expit((mu - e) / (T + 1e-12)) formed inside the density pass:
+        // the same value as expit(-(e - mu) / (T + 1e-12)), one launch less
+        CPPHF_TRY(dm_dens_occ(V, e_occ, mu_fin, K->T + 1.0e-12, occ, Pout, nk, nb, st));
         if (project) {
             CPPHF_TRY(call_project(project, puser, Pout, K, st));
             CPPHF_TRY(hermitize(Pout, Pout, nk, nb, st));
@@ -927,19 +866,6 @@ int solve_scf(const cpphf_kernel* K, const cpphf_scf_config* cfg, const double2*
     bool converged = false;
     int64_t k = 0;
     const double wsum = std::max(K->weight_sum, 1.0e-30);
-    const unsigned tgrid = [&] {
-        const int64_t teams = nb <= kTeamWarpMaxNb ? kWarpTeams : 1;
-        return (unsigned)std::max<int64_t>(1, std::min<int64_t>((nk + teams - 1) / teams, kDmMaxPartials));
-    }();
-    const bool warp = nb <= kTeamWarpMaxNb;
-    const size_t per = (sizeof(double2) * team_mat_elems(nb) * 2 + 15) & ~(size_t)15;
-    const size_t rsmem = per * (warp ? kWarpTeams : 1);
-    static std::once_flag attrs;
-    std::call_once(attrs, [] {
-        raise_smem(k_scf_residuals<true>);
-        raise_smem(k_scf_residuals<false>);
-    });
-
     // acceleration state
     const int acc = cfg->acceleration;
     const int64_t nel = nk * (int64_t)nb * nb;
@@ -984,12 +910,8 @@ int solve_scf(const cpphf_kernel* K, const cpphf_scf_config* cfg, const double2*
             if (dm_small_supported(nb))
                 CPPHF_TRY(scf_small_residuals(F, D, Pn, K->w2d, nk, nb, S, comm_out, fuse_mix ? D : nullptr,
                                               cfg->mixing, st));
-            else if (warp)
-                k_scf_residuals<true><<<tgrid, 32 * kWarpTeams, rsmem, st>>>(F, D, Pn, K->w2d, nk, nb, S, comm_out);
             else
-                k_scf_residuals<false><<<tgrid, kCtaTeamThreadsDense, rsmem, st>>>(F, D, Pn, K->w2d, nk, nb, S,
-                                                                                    comm_out);
-            CPPHF_LAUNCH_CHECK("scf residuals");
+                CPPHF_TRY(scf_mma_residuals(F, D, Pn, K->w2d, nk, nb, S, comm_out, st));
             return CPPHF_OK;
         };
         const int lw = low ? 1 : 0;
@@ -1189,9 +1111,7 @@ int density_from_fock(const double2* F, const double* w, int64_t nk1, int64_t nk
         CPPHF_TRY(mu_solve(e_occ, w, nk, nb, n_e, nullptr, T, 30, 0, &mu2[1], mws, mb, st));
         mu = &mu2[1];
     }
-    k_fermi<<<grid_for(nk * nb, 256), 256, 0, st>>>(e_occ, mu, T, occ, nk * nb);
-    CPPHF_LAUNCH_CHECK("fermi");
-    CPPHF_TRY(dm_density(V, occ, P, nk, (int)nb, st));
+    CPPHF_TRY(dm_dens_occ(V, e_occ, mu, T + 1.0e-12, occ, P, nk, (int)nb, st));
     CPPHF_CUDA(cudaMemcpyAsync(mu_out, mu, sizeof(double), cudaMemcpyDeviceToDevice, st));
     return CPPHF_OK;
 }
