@@ -8,7 +8,7 @@
 // (one product is 10.9 GFLOP, 0.30 ms at the FP64 rate), before -> now, ms:
 // density 1.47 -> 0.26 (half a product), trial 9.7 -> 1.02 (an inverse and a
 // product), retraction 9.9 -> 0.42, rotation + gradient 2.9 -> 0.91 (two).
-// At nb = 9, the most padded size, on 96 x 96, us: trial 165 -> 143, retraction
+// At nb = 9, the most padded size, on 96 x 96, us: trial 74 -> 58, retraction
 // 69 -> 30, rotation + gradient 44 -> 42, density 22 -> 20.
 #include "common.cuh"
 #include "dm.cuh"

@@ -17,20 +17,23 @@
 // Line lengths with a register codelet (fft_reg.cuh: 1..6, 8, 9, 12, 16, 18,
 // 24, 32, 36, 48, 64, 72, 96, 128, 144, 192, 256, 288) run the four-step
 // transform with global loads/stores straight from/to registers and one
-// shared-memory transpose per direction; any other length runs the generic
-// out-of-place Stockham stages of fft.cuh.
+// shared-memory transpose per direction; other lengths run the mixed-radix passes
+// of exchange_smooth.cu in complex128 (also for zero-padded fields) and the
+// out-of-place Stockham stages of fft.cuh in complex64.
 #include "common.cuh"
 #include "exchange.cuh"
 #include "fft.cuh"
 #include "fft_reg.cuh"
 #include "bulk.cuh"
 #include "exchange_pipe.cuh"
+#include "exchange_smooth.cuh"
 
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
 #include <string>
+#include <type_traits>
 
 namespace cpphf {
 
@@ -870,15 +873,20 @@ int pass_rows_fwd(const double2* P, const double2* refP, Cx* T, const ExchangeGe
 #undef X
         default: break;
     }
-    FftPlan1D pl;
-    if (!make_plan(g.n1, pl)) return fail(CPPHF_ERR_INVALID, "exchange: mesh size has too many prime factors");
-    Gen<Cx>::attrs();
-    const Launch L = plan_launch(g.n1, g.C, sizeof(Cx), g.n1, true);
-    if (L.smem > kSmemMax) return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
-    k_rows_fwd_g<Cx><<<dim3(g.n0, L.nchunk), cap_threads(k_rows_fwd_g<Cx>, L.threads), L.smem, st>>>(P, refP, T, g,
-                                                                                                     pl, L.CB);
-    CPPHF_LAUNCH_CHECK("exchange rows forward");
-    return CPPHF_OK;
+    if constexpr (std::is_same_v<Cx, double2>) {
+        return smooth_rows_fwd(P, refP, T, g, st);
+    } else {
+        FftPlan1D pl;
+        if (!make_plan(g.n1, pl)) return fail(CPPHF_ERR_INVALID, "exchange: mesh size has too many prime factors");
+        Gen<Cx>::attrs();
+        const Launch L = plan_launch(g.n1, g.C, sizeof(Cx), g.n1, true);
+        if (L.smem > kSmemMax)
+            return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
+        k_rows_fwd_g<Cx><<<dim3(g.n0, L.nchunk), cap_threads(k_rows_fwd_g<Cx>, L.threads), L.smem, st>>>(P, refP, T, g,
+                                                                                                         pl, L.CB);
+        CPPHF_LAUNCH_CHECK("exchange rows forward");
+        return CPPHF_OK;
+    }
 }
 
 template <class Cx>
@@ -890,15 +898,20 @@ int pass_cols(Cx* T, const double2* VR, const ExchangeGeom& g, int vmode, cudaSt
 #undef X
         default: break;
     }
-    FftPlan1D pl;
-    if (!make_plan(g.n0, pl)) return fail(CPPHF_ERR_INVALID, "exchange: mesh size has too many prime factors");
-    Gen<Cx>::attrs();
-    const Launch L = plan_launch(g.n0, g.C, sizeof(Cx), g.n0, true);
-    if (L.smem > kSmemMax) return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
-    k_cols_conv_g<Cx><<<dim3(g.n1, L.nchunk), cap_threads(k_cols_conv_g<Cx>, L.threads), L.smem, st>>>(T, VR, g, pl,
-                                                                                                       L.CB, vmode);
-    CPPHF_LAUNCH_CHECK("exchange columns convolve");
-    return CPPHF_OK;
+    if constexpr (std::is_same_v<Cx, double2>) {
+        return smooth_cols(T, VR, g, vmode, st);
+    } else {
+        FftPlan1D pl;
+        if (!make_plan(g.n0, pl)) return fail(CPPHF_ERR_INVALID, "exchange: mesh size has too many prime factors");
+        Gen<Cx>::attrs();
+        const Launch L = plan_launch(g.n0, g.C, sizeof(Cx), g.n0, true);
+        if (L.smem > kSmemMax)
+            return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
+        k_cols_conv_g<Cx><<<dim3(g.n1, L.nchunk), cap_threads(k_cols_conv_g<Cx>, L.threads), L.smem, st>>>(T, VR, g, pl,
+                                                                                                           L.CB, vmode);
+        CPPHF_LAUNCH_CHECK("exchange columns convolve");
+        return CPPHF_OK;
+    }
 }
 
 template <class Cx>
@@ -910,15 +923,20 @@ int pass_rows_inv(const Cx* T, double2* Sigma, const ExchangeGeom& g, double sca
 #undef X
         default: break;
     }
-    FftPlan1D pl;
-    if (!make_plan(g.n1, pl)) return fail(CPPHF_ERR_INVALID, "exchange: mesh size has too many prime factors");
-    Gen<Cx>::attrs();
-    const Launch L = plan_launch(g.n1, g.C, sizeof(Cx), g.n1, true);
-    if (L.smem > kSmemMax) return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
-    k_rows_inv_g<Cx><<<dim3(g.n0, L.nchunk), cap_threads(k_rows_inv_g<Cx>, L.threads), L.smem, st>>>(T, Sigma, g, pl,
-                                                                                                     L.CB, scale);
-    CPPHF_LAUNCH_CHECK("exchange rows inverse");
-    return CPPHF_OK;
+    if constexpr (std::is_same_v<Cx, double2>) {
+        return smooth_rows_inv(T, Sigma, g, scale, st);
+    } else {
+        FftPlan1D pl;
+        if (!make_plan(g.n1, pl)) return fail(CPPHF_ERR_INVALID, "exchange: mesh size has too many prime factors");
+        Gen<Cx>::attrs();
+        const Launch L = plan_launch(g.n1, g.C, sizeof(Cx), g.n1, true);
+        if (L.smem > kSmemMax)
+            return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
+        k_rows_inv_g<Cx><<<dim3(g.n0, L.nchunk), cap_threads(k_rows_inv_g<Cx>, L.threads), L.smem, st>>>(T, Sigma, g, pl,
+                                                                                                         L.CB, scale);
+        CPPHF_LAUNCH_CHECK("exchange rows inverse");
+        return CPPHF_OK;
+    }
 }
 
 template <class Cx>
@@ -968,6 +986,8 @@ int exchange(const double2* P, const double2* refP, const double2* VR, double2* 
     ExchangeGeom g;
     g.n0 = (int)nk1;
     g.n1 = (int)nk2;
+    g.s0 = g.n0;
+    g.s1 = g.n1;
     g.nb = (int)nb;
     g.hcp = hcp ? 1 : 0;
     g.C = hcp ? (int)(nb * (nb + 1) / 2) : (int)(nb * nb);
@@ -985,6 +1005,29 @@ int exchange(const double2* P, const double2* refP, const double2* VR, double2* 
         return launch_exchange<float2>(P, refP, VR, Sigma, static_cast<float2*>(workspace), g, st, kColsVR);
     double2* T = hcp ? static_cast<double2*>(workspace) : Sigma;
     return launch_exchange<double2>(P, refP, VR, Sigma, T, g, st, kColsVR);
+}
+
+bool exchange_padded_supported(int64_t n0, int64_t n1, int64_t nb) {
+    if (n0 > 65535 || n1 > 65535 || (split_of((int)n0).n1 && split_of((int)n1).n1)) return false;
+    const int C = (int)(nb * nb);
+    return smooth_supported((int)n0, C) && smooth_supported((int)n1, C);
+}
+
+int exchange_padded(double2* X, const double2* VR, double2* T, int64_t n0, int64_t n1, int64_t s0, int64_t s1,
+                    int64_t nb, int64_t dv, cudaStream_t st) {
+    ExchangeGeom g;
+    g.n0 = (int)n0;
+    g.n1 = (int)n1;
+    g.s0 = (int)s0;
+    g.s1 = (int)s1;
+    g.nb = (int)nb;
+    g.hcp = 0;
+    g.C = g.Ct = (int)(nb * nb);
+    g.dv = dv == 1 ? 1 : g.C;
+    g.shift = 0;
+    CPPHF_TRY(smooth_rows_fwd(X, nullptr, T, g, st));
+    CPPHF_TRY(smooth_cols(T, VR, g, kSmoothVR, st));
+    return smooth_rows_inv(T, X, g, -1.0 / ((double)n0 * (double)n1), st);
 }
 
 namespace {
@@ -1022,6 +1065,8 @@ ExchangeGeom full_geom(int64_t nk1, int64_t nk2, int64_t nb, int64_t dv) {
     ExchangeGeom g;
     g.n0 = (int)nk1;
     g.n1 = (int)nk2;
+    g.s0 = g.n0;
+    g.s1 = g.n1;
     g.nb = (int)nb;
     g.hcp = 0;
     g.C = (int)(nb * nb);

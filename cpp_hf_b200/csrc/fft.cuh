@@ -1,4 +1,4 @@
-// Generic shared-memory batched 1-D FFT on a tile of n points x CB channels,
+// Generic shared-memory batched 1-D FFT (the complex64 exchange) on a tile of n points x CB channels,
 // for line lengths that have no register codelet (fft_reg.cuh).
 //
 // The tile is row-major [n][CB] complex in shared memory (channel fastest).  A

@@ -638,6 +638,8 @@ int build_fock_packed(const cpphf_kernel* K, const double2* P, double2* Sigma, d
     ExchangeGeom g;
     g.n0 = (int)K->nk1;
     g.n1 = (int)K->nk2;
+    g.s0 = g.n0;
+    g.s1 = g.n1;
     g.nb = (int)K->nb;
     g.hcp = 0;
     g.shift = 0;

@@ -46,7 +46,7 @@ struct SlPlan {
 // rho (x, y, i, a, j, b) -> extended field (ox + x, oy + y, channel of (slot, a, b))
 __global__ void k_sl_scatter(const double2* __restrict__ rho, double2* __restrict__ buf,
                              const SlEntry* __restrict__ ent, int n_ent, const int* __restrict__ goff, int nkx,
-                             int nky, int nG, int orb, int NY, int C, int nbf, int kq) {
+                             int nky, int nG, int orb, int ld, int C, int nbf, int kq) {
     const int64_t blk = (int64_t)nkx * nky * orb * orb;
     const int64_t total = (int64_t)n_ent * blk;
     const int64_t D = (int64_t)nG * orb;
@@ -63,14 +63,14 @@ __global__ void k_sl_scatter(const double2* __restrict__ rho, double2* __restric
         const int ox = nkx * goff[2 * en.i], oy = nky * goff[2 * en.i + 1];
         const double2 v = rho[(((int64_t)x * nky + y) * D + (int64_t)en.i * orb + a) * D + (int64_t)en.j * orb + b];
         const int c = ((en.slot / kq) * orb + a) * nbf + (en.slot % kq) * orb + b;
-        buf[((int64_t)(ox + x) * NY + (oy + y)) * C + c] = v;
+        buf[((int64_t)(ox + x) * ld + (oy + y)) * C + c] = v;
     }
 }
 
 // extended field -> sigma blocks (and their conjugate transposes for partners)
 __global__ void k_sl_gather(const double2* __restrict__ buf, double2* __restrict__ sigma,
                             const SlEntry* __restrict__ ent, int n_ent, const int* __restrict__ goff, int nkx,
-                            int nky, int nG, int orb, int NY, int C, int nbf, int kq) {
+                            int nky, int nG, int orb, int ld, int C, int nbf, int kq) {
     const int64_t blk = (int64_t)nkx * nky * orb * orb;
     const int64_t total = (int64_t)n_ent * blk;
     const int64_t D = (int64_t)nG * orb;
@@ -86,7 +86,7 @@ __global__ void k_sl_gather(const double2* __restrict__ buf, double2* __restrict
         const SlEntry en = ent[e];
         const int ox = nkx * goff[2 * en.i], oy = nky * goff[2 * en.i + 1];
         const int c = ((en.slot / kq) * orb + a) * nbf + (en.slot % kq) * orb + b;
-        const double2 v = buf[((int64_t)(ox + x) * NY + (oy + y)) * C + c];
+        const double2 v = buf[((int64_t)(ox + x) * ld + (oy + y)) * C + c];
         const int64_t kxy = (int64_t)x * nky + y;
         sigma[(kxy * D + (int64_t)en.i * orb + a) * D + (int64_t)en.j * orb + b] = v;
         if (en.partner) sigma[(kxy * D + (int64_t)en.j * orb + b) * D + (int64_t)en.i * orb + a] = cconj(v);
@@ -241,17 +241,32 @@ int superlattice_streamed(const double2* rho, const double2* VR, const double2* 
     const int64_t D = nG * orb;
     CPPHF_CUDA(cudaMemsetAsync(sigma, 0, sizeof(double2) * (size_t)nkx * nky * D * D, st));
     const double2* vr = VRo ? VRo : VR;
+    // the tiles cover the first s0 x s1 points; the rest of the extended grid is
+    // padding, which the mixed-radix passes neither store nor transform.  Grids with
+    // codelets on both axes keep the codelet passes: 118 us against 128 with the
+    // padded ones at 288 x 288, 4 plane waves, and equal at 144 and 72.
+    int64_t s0 = 0, s1 = 0;
+    for (int64_t i = 0; i < nG; ++i) {
+        s0 = std::max(s0, (g_a_off[2 * i] + 1) * nkx);
+        s1 = std::max(s1, (g_a_off[2 * i + 1] + 1) * nky);
+    }
+    const bool padded = exchange_padded_supported(NX, NY, pl.nbf);
+    const size_t in_bytes = padded ? sizeof(double2) * (size_t)s0 * s1 * pl.C : fbytes;
+    const int row = (int)(padded ? s1 : NY);
     for (size_t bi = 0; bi + 1 < pl.batch_start.size(); ++bi) {
         const int e0 = pl.batch_start[bi], e1 = pl.batch_start[bi + 1];
         const int n_ent = e1 - e0;
         const int64_t work = (int64_t)n_ent * nkx * nky * orb * orb;
-        CPPHF_CUDA(cudaMemsetAsync(buf_in, 0, fbytes, st));
+        CPPHF_CUDA(cudaMemsetAsync(buf_in, 0, in_bytes, st));
         k_sl_scatter<<<grid_for_n(work), 256, 0, st>>>(rho, buf_in, d_ent + e0, n_ent, d_goff, (int)nkx, (int)nky,
-                                                      (int)nG, (int)orb, (int)NY, pl.C, pl.nbf, pl.kq);
+                                                      (int)nG, (int)orb, row, pl.C, pl.nbf, pl.kq);
         CPPHF_LAUNCH_CHECK("superlattice scatter");
-        CPPHF_TRY(exchange(buf_in, nullptr, vr, buf_out, NX, NY, pl.nbf, pl.dv, 0, 0, 64, nullptr, 0, st));
-        k_sl_gather<<<grid_for_n(work), 256, 0, st>>>(buf_out, sigma, d_ent + e0, n_ent, d_goff, (int)nkx, (int)nky,
-                                                     (int)nG, (int)orb, (int)NY, pl.C, pl.nbf, pl.kq);
+        if (padded)
+            CPPHF_TRY(exchange_padded(buf_in, vr, buf_out, NX, NY, s0, s1, pl.nbf, pl.dv, st));
+        else
+            CPPHF_TRY(exchange(buf_in, nullptr, vr, buf_out, NX, NY, pl.nbf, pl.dv, 0, 0, 64, nullptr, 0, st));
+        k_sl_gather<<<grid_for_n(work), 256, 0, st>>>(padded ? buf_in : buf_out, sigma, d_ent + e0, n_ent, d_goff, (int)nkx, (int)nky,
+                                                     (int)nG, (int)orb, row, pl.C, pl.nbf, pl.kq);
         CPPHF_LAUNCH_CHECK("superlattice gather");
     }
     // the pageable copies above are staged before cudaMemcpyAsync returns, so
