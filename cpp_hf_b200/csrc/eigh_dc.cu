@@ -40,6 +40,13 @@ namespace cpphf {
 namespace {
 
 constexpr double kEps = 2.220446049250313e-16;
+// Squared norms below this are zero at working precision (the matrix is scaled to
+// O(1)); their square roots would have lost their digits to underflow.
+constexpr double kTinyNorm2 = 1e-290;
+__device__ __forceinline__ double modulus(double2 x) {
+    const double m2 = fma(x.x, x.x, x.y * x.y);
+    return m2 > kTinyNorm2 ? sqrt(m2) : 0.0;
+}
 constexpr int kSecularMaxIter = 60;  // safeguarded: a bisection of the bracket at worst
 
 template <int NE>
@@ -229,7 +236,8 @@ __global__ void __launch_bounds__(DcGeo<NE>::NT, DcGeo<NE>::BLOCKS)
             xn2 += __shfl_xor_sync(quad, xn2, 2);
             const int src = (lane & 28) + ((k + 1) & 3);
             x0 = mk(__shfl_sync(quad, x0.x, src), __shfl_sync(quad, x0.y, src));
-            const double ax0 = sqrt(fma(x0.x, x0.x, x0.y * x0.y)), xn = sqrt(xn2);
+            const double ax0 = modulus(x0), xn = sqrt(xn2);
+            const bool some = xn2 > kTinyNorm2;
             const double2 ph = ax0 > 0.0 ? mk(x0.x / ax0, x0.y / ax0) : mk(1.0, 0.0);
             double2* Uk = s.U + (size_t)k * (n - 1) - (size_t)k * (k - 1) / 2 - (k + 1);
 #pragma unroll
@@ -242,8 +250,8 @@ __global__ void __launch_bounds__(DcGeo<NE>::NT, DcGeo<NE>::BLOCKS)
                 }
             }
             if (q == 0) {
-                s.beta[k] = xn > 0.0 ? 1.0 / (xn * (xn + ax0)) : 0.0;
-                s.sub[k] = xn > 0.0 ? mk(-ph.x * xn, -ph.y * xn) : x0;
+                s.beta[k] = some ? 1.0 / (xn * (xn + ax0)) : 0.0;
+                s.sub[k] = some ? mk(-ph.x * xn, -ph.y * xn) : x0;
             }
         }
         __syncthreads();
@@ -302,12 +310,12 @@ __global__ void __launch_bounds__(DcGeo<NE>::NT, DcGeo<NE>::BLOCKS)
     double2* delta = s.ub[0];
     if (q == 0 && j < n) {
         double ej = 0.0;
-        if (j + 1 < n) ej = sqrt(fma(s.sub[j].x, s.sub[j].x, s.sub[j].y * s.sub[j].y));
+        if (j + 1 < n) ej = modulus(s.sub[j]);
         s.e[j] = ej;
         double2 x = mk(1.0, 0.0);
         if (j > 0) {
             const double2 v = s.sub[j - 1];
-            const double m = sqrt(fma(v.x, v.x, v.y * v.y));
+            const double m = modulus(v);
             if (m > 0.0) x = mk(v.x / m, v.y / m);
         }
         delta[j] = x;

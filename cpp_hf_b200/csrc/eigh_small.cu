@@ -1,8 +1,9 @@
 // Batched Hermitian eigendecomposition for small matrices (nb <= 8):
 // Householder reduction to real tridiagonal form followed by implicit QL
-// iterations, GS = (nb rounded up to 2, 4 or 8) lanes per matrix, everything in
-// registers (replaces Eigen's SelfAdjointEigenSolver in cpp_hf linalg.hpp:39-66,
-// which takes the same tridiagonal + QL route).
+// iterations, everything in registers (replaces Eigen's SelfAdjointEigenSolver in
+// cpp_hf linalg.hpp:39-66, which takes the same tridiagonal + QL route): eight
+// lanes per matrix for small batches of nb = 5..8, one thread per matrix
+// otherwise (k_eigh_thread, below).
 //
 // Lane r of a group owns column r of A and row r of the accumulated unitary Z.
 //  1. Reduction, k = 0 .. nb-3: lane k forms the reflector H = I - beta u u^H
@@ -26,6 +27,7 @@
 #include "eigh.cuh"
 
 #include <cstdlib>
+#include <mutex>
 
 namespace cpphf {
 
@@ -34,10 +36,15 @@ namespace {
 constexpr int kHqlThreads = 128;
 constexpr int kQlMaxIter = 60;  // QL iterations per eigenvalue before giving up
 
-template <int NB>
-struct HqlGeo {
-    static constexpr int GS = NB <= 2 ? 2 : (NB <= 4 ? 4 : 8);
-};
+constexpr int kGroup = 8;  // lanes per matrix of the group form
+
+// Squared norms below this are zero at working precision (the matrices are scaled
+// to O(1)); their square roots would have lost their digits to underflow.
+constexpr double kTinyNorm2 = 1e-290;
+__device__ __forceinline__ double modulus(double2 x) {
+    const double m2 = fma(x.x, x.x, x.y * x.y);
+    return m2 > kTinyNorm2 ? sqrt(m2) : 0.0;
+}
 
 template <int GS>
 __device__ __forceinline__ double group_sum(double v, unsigned mask) {
@@ -50,16 +57,11 @@ __device__ __forceinline__ double2 shfl2(double2 v, int src, unsigned mask) {
     return mk(__shfl_sync(mask, v.x, src), __shfl_sync(mask, v.y, src));
 }
 
-// four CTAs per SM (<= 128 registers, a few spilled): on the Fock matrices of
-// an SCF solve (192 x 192, nb = 8) 194 us per call against 220 us at three CTAs
-// without spills (on random Hermitian matrices three CTAs are 4 % faster).
-// Splitting the kernel after the reduction (a QL kernel at 96 registers and
-// five CTAs per SM, the tridiagonal and Z handed over through V) was slower:
-// the QL is bound by its instruction count more than by latency.
+// four CTAs per SM (<= 128 registers, a few spilled)
 template <int NB>
 __global__ void __launch_bounds__(kHqlThreads, 4) k_eigh_hql(const double2* __restrict__ M, double* __restrict__ w,
                                                           double2* __restrict__ Vout, int64_t batch, int mode) {
-    constexpr int GS = HqlGeo<NB>::GS;
+    constexpr int GS = kGroup;
     const int lane = threadIdx.x & 31;
     const int r = lane % GS;
     const int base = lane - r;
@@ -111,9 +113,8 @@ __global__ void __launch_bounds__(kHqlThreads, 4) k_eigh_hql(const double2* __re
 #pragma unroll
             for (int i = kk + 1; i < NB; ++i) xn2 += a[i].x * a[i].x + a[i].y * a[i].y;
             const double2 x0 = a[kk + 1];
-            // entries are O(1) after the scaling, so the plain modulus cannot overflow
-            const double ax0 = sqrt(fma(x0.x, x0.x, x0.y * x0.y));
-            const double xn = sqrt(xn2);
+            const double ax0 = modulus(x0);
+            const double xn = xn2 > kTinyNorm2 ? sqrt(xn2) : 0.0;
 #pragma unroll
             for (int i = 0; i < NB; ++i) ul[i] = mk(0.0, 0.0);
             if (xn > 0.0) {
@@ -202,7 +203,7 @@ __global__ void __launch_bounds__(kHqlThreads, 4) k_eigh_hql(const double2* __re
     for (int i = 0; i < NB; ++i) {
         z[i] = cmul(z[i], delta);
         if (i + 1 < NB) {
-            const double m = sqrt(fma(sub[i].x, sub[i].x, sub[i].y * sub[i].y));
+            const double m = modulus(sub[i]);
             e[i] = m;
             if (m > 0.0) {
                 const double im = 1.0 / m;
@@ -339,17 +340,318 @@ __global__ void __launch_bounds__(kHqlThreads, 4) k_eigh_hql(const double2* __re
     }
 }
 
+// ---------------------------------------------------------------------------
+// Large batches: one thread per matrix, the same reduction and QL.
+//
+// In the group form every lane repeats the scalar QL recurrence (about forty FP64
+// instructions a rotation) to rotate its one row of Z; here a thread runs it once
+// and rotates all NB rows of the real eigenvector matrix of the tridiagonal, so
+// the FP64 work of a matrix falls to about a third.  The lower triangle of A,
+// later Z, fills the registers (two warps per scheduler); the reflectors, scaled
+// so that H = I - u u^H, and the phases wait in shared memory.  The columns of Z
+// are sorted in registers and transformed two at a time through a padded staging
+// tile, so that V is written in whole 32-byte sectors.  The work of a warp is one
+// long chain (255 registers, a few spilled at nb = 8), which bounds it up to two
+// warps per scheduler; the FP64 pipe does beyond that.  36864 matrices of nb = 8:
+// 249 us in groups, 81 us here.
+// ---------------------------------------------------------------------------
+constexpr int kThreadCta = 64;
+
+template <int NB>
+struct ThreadGeo {
+    static constexpr int NU = NB * (NB - 1) / 2;               // reflector entries u_k[k+1..NB-1]
+    static constexpr int WORDS = 2 * NU + 2 * NB;              // doubles per matrix in shared memory
+    static constexpr int STG = 2 * NB + 1;                     // staging stride of a matrix, double2
+    static constexpr size_t kSmem = sizeof(double) * WORDS * kThreadCta + sizeof(double2) * STG * kThreadCta;
+};
+
+template <int NB>
+__global__ void __launch_bounds__(kThreadCta, 4)
+    k_eigh_thread(const double2* __restrict__ M, double* __restrict__ w, double2* __restrict__ Vout, int64_t batch,
+                  int mode) {
+    using G = ThreadGeo<NB>;
+    extern __shared__ __align__(16) unsigned char raw[];
+    double* sm = reinterpret_cast<double*>(raw) + threadIdx.x;  // word i of the thread at sm[i * kThreadCta]
+    const int lane = threadIdx.x & 31, wbase = threadIdx.x - lane;
+    double2* stg = reinterpret_cast<double2*>(raw + sizeof(double) * G::WORDS * kThreadCta) + (size_t)wbase * G::STG;
+    const int64_t k0 = (int64_t)blockIdx.x * kThreadCta + wbase;  // first matrix of the warp
+    if (k0 >= batch) return;
+    const int64_t k = min(k0 + lane, batch - 1);  // spare lanes repeat the last matrix
+    auto put = [&](int i, double2 v) {
+        sm[(2 * i) * kThreadCta] = v.x;
+        sm[(2 * i + 1) * kThreadCta] = v.y;
+    };
+    auto get = [&](int i) { return mk(sm[(2 * i) * kThreadCta], sm[(2 * i + 1) * kThreadCta]); };
+    constexpr auto uoff = [](int kk) { return kk * (NB - 1) - kk * (kk - 1) / 2 - (kk + 1); };  // entry of u_kk[i]: + i
+
+    double d[NB], e[NB];
+    int ex = 0;
+    {
+        // lower triangle of herm(M) or herm(i M), scaled by a power of two
+        double2 a[NB][NB];
+        const double2* Mk = M + (size_t)k * NB * NB;
+        double amax = 0.0;
+#pragma unroll
+        for (int i = 0; i < NB; ++i)
+#pragma unroll
+            for (int j = 0; j < NB; ++j) {
+                double2 x = Mk[i * NB + j];
+                if (mode == 1) x = mk(-x.y, x.x);
+                if (j < i) {
+                    a[i][j] = x;  // finished when row j's entry (j, i) was read before
+                    a[i][j] = mk(0.5 * (x.x + a[j][i].x), 0.5 * (x.y - a[j][i].y));
+                } else {
+                    a[i][j] = x;
+                }
+            }
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            a[i][i].y = 0.0;
+#pragma unroll
+            for (int j = 0; j <= i; ++j) amax = fmax(amax, fmax(fabs(a[i][j].x), fabs(a[i][j].y)));
+        }
+        if (amax > 0.0 && isfinite(amax)) frexp(amax, &ex);
+        const double sc = ldexp(1.0, -ex);
+        // 2^-ex may be subnormal or infinite at the ends of the range: scale in two steps there
+        const bool two = !(fabs(sc) >= 2.3e-308 && isfinite(sc));
+#pragma unroll
+        for (int i = 0; i < NB; ++i)
+#pragma unroll
+            for (int j = 0; j <= i; ++j) {
+                if (two)
+                    a[i][j] = mk(ldexp(a[i][j].x, -ex), ldexp(a[i][j].y, -ex));
+                else
+                    a[i][j] = cscale(a[i][j], sc);
+            }
+        // ---- 1. reduction ----
+        double2 sub[NB];
+#pragma unroll
+        for (int kk = 0; kk + 2 < NB; ++kk) {
+            double xn2 = 0.0;
+#pragma unroll
+            for (int i = kk + 1; i < NB; ++i) xn2 += a[i][kk].x * a[i][kk].x + a[i][kk].y * a[i][kk].y;
+            const double2 x0 = a[kk + 1][kk];
+            const double ax0 = modulus(x0), xn = sqrt(xn2);
+            const bool on = xn2 > kTinyNorm2;
+            const double iax = ax0 > 0.0 ? 1.0 / ax0 : 0.0;
+            const double2 ph = ax0 > 0.0 ? mk(x0.x * iax, x0.y * iax) : mk(1.0, 0.0);
+            // beta = 1 / (xn (xn + ax0)); u is scaled by its square root
+            const double rb = on ? rsqrt(xn * (xn + ax0)) : 0.0;
+            sub[kk] = on ? mk(-ph.x * xn, -ph.y * xn) : x0;
+            double2 u[NB], p[NB];
+#pragma unroll
+            for (int i = kk + 1; i < NB; ++i) {
+                u[i] = i == kk + 1 ? mk((x0.x + ph.x * xn) * rb, (x0.y + ph.y * xn) * rb) : cscale(a[i][kk], rb);
+                put(uoff(kk) + i, u[i]);
+            }
+            double K = 0.0;
+#pragma unroll
+            for (int i = kk + 1; i < NB; ++i) {
+                double2 s = cscale(u[i], a[i][i].x);
+#pragma unroll
+                for (int j = kk + 1; j < i; ++j) cfma(s, a[i][j], u[j]);
+#pragma unroll
+                for (int j = i + 1; j < NB; ++j) cfma(s, cconj(a[j][i]), u[j]);
+                p[i] = s;
+                K += u[i].x * s.x + u[i].y * s.y;
+            }
+            K *= 0.5;
+#pragma unroll
+            for (int i = kk + 1; i < NB; ++i) p[i] = mk(p[i].x - K * u[i].x, p[i].y - K * u[i].y);
+#pragma unroll
+            for (int i = kk + 1; i < NB; ++i)
+#pragma unroll
+                for (int j = kk + 1; j <= i; ++j) {
+                    a[i][j] = csub(a[i][j], cmulc(u[i], p[j]));
+                    a[i][j] = csub(a[i][j], cmulc(p[i], u[j]));
+                }
+        }
+        if constexpr (NB >= 2) sub[NB - 2] = a[NB - 1][NB - 2];
+        // ---- 2. real tridiagonal ----
+        double2 delta = mk(1.0, 0.0);
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            d[i] = a[i][i].x;
+            put(G::NU + i, delta);
+            e[i] = 0.0;
+            if (i + 1 < NB) {
+                const double m = modulus(sub[i]);
+                e[i] = m;
+                if (m > 0.0) {
+                    const double im = 1.0 / m;
+                    delta = cmul(delta, mk(sub[i].x * im, sub[i].y * im));
+                }
+            }
+        }
+    }
+
+    // ---- 3. implicit QL on (d, e) with the real eigenvectors z[row][col] ----
+    double z[NB][NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i)
+#pragma unroll
+        for (int j = 0; j < NB; ++j) z[i][j] = i == j ? 1.0 : 0.0;
+    constexpr double kEps = 2.220446049250313e-16;
+#pragma unroll
+    for (int l = 0; l < NB; ++l) {
+        for (int iter = 0; iter < kQlMaxIter; ++iter) {
+            int m = NB - 1;
+#pragma unroll
+            for (int i = NB - 2; i >= l; --i)
+                if (fabs(e[i]) <= kEps * (fabs(d[i]) + fabs(d[i + 1]))) m = i;
+            if (m == l) break;
+            double dm = d[NB - 1];
+#pragma unroll
+            for (int j = l; j < NB; ++j)
+                if (j == m) dm = d[j];
+            const double el = e[l], t = (l + 1 < NB ? d[l + 1 < NB ? l + 1 : l] : 0.0) - d[l], u2 = 2.0 * el;
+            const double den = t + copysign(sqrt(fma(t, t, u2 * u2)), t);
+            double g;
+            if (den != 0.0) {
+                g = dm - d[l] + el * u2 / den;
+            } else {
+                g = t / u2;
+                g = dm - d[l] + el / (g + copysign(sqrt(fma(g, g, 1.0)), g));
+            }
+            double s = 1.0, c = 1.0, p = 0.0;
+            bool under = false;
+#pragma unroll
+            for (int i = NB - 2; i >= l; --i) {
+                if (i < m && !under) {
+                    const double f = s * e[i], b = c * e[i], q = fma(f, f, g * g);
+                    if (q == 0.0) {
+                        e[i + 1] = 0.0;
+                        d[i + 1] -= p;
+                        under = true;
+                    } else {
+                        const double rinv = rsqrt(q);
+                        e[i + 1] = q * rinv;
+                        s = f * rinv;
+                        c = g * rinv;
+                        g = d[i + 1] - p;
+                        const double tt = (d[i] - g) * s + 2.0 * c * b;
+                        p = s * tt;
+                        d[i + 1] = g + p;
+                        g = c * tt - b;
+#pragma unroll
+                        for (int r = 0; r < NB; ++r) {
+                            const double zi = z[r][i], z1 = z[r][i + 1];
+                            z[r][i + 1] = s * zi + c * z1;
+                            z[r][i] = c * zi - s * z1;
+                        }
+                    }
+                }
+            }
+            if (!under) {
+                d[l] -= p;
+                e[l] = g;
+            }
+#pragma unroll
+            for (int j = l; j < NB; ++j)
+                if (j == m) e[j] = 0.0;
+        }
+    }
+
+    // ---- 4. ascending order: odd-even transposition of (d, columns), stable ----
+#pragma unroll
+    for (int round = 0; round < NB; ++round)
+#pragma unroll
+        for (int i = round & 1; i + 1 < NB; i += 2) {
+            const bool sw = d[i + 1] < d[i];
+            const double t = d[i];
+            d[i] = sw ? d[i + 1] : t;
+            d[i + 1] = sw ? t : d[i + 1];
+#pragma unroll
+            for (int r = 0; r < NB; ++r) {
+                const double x = z[r][i];
+                z[r][i] = sw ? z[r][i + 1] : x;
+                z[r][i + 1] = sw ? x : z[r][i + 1];
+            }
+        }
+    const int cnt = (int)min((int64_t)32, batch - k0);
+    if (lane < cnt) {
+#pragma unroll
+        for (int i = 0; i < NB; ++i) w[(size_t)k * NB + i] = ldexp(d[i], ex);
+    }
+    // ---- 5. V = H_0 .. H_{NB-3} diag(delta) Z, two columns at a time ----
+#pragma unroll
+    for (int c0 = 0; c0 < NB; c0 += 2) {
+        constexpr int W = 2;
+        const int nc = NB - c0 < W ? NB - c0 : W;
+        double2 v[W][NB];
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            const double2 dl = get(G::NU + i);
+#pragma unroll
+            for (int c = 0; c < W; ++c) v[c][i] = cscale(dl, z[i][c0 + c < NB ? c0 + c : c0]);
+        }
+#pragma unroll
+        for (int kk = NB - 3; kk >= 0; --kk) {
+            double2 t[W];
+#pragma unroll
+            for (int c = 0; c < W; ++c) t[c] = mk(0.0, 0.0);
+#pragma unroll
+            for (int i = kk + 1; i < NB; ++i) {
+                const double2 u = get(uoff(kk) + i);
+#pragma unroll
+                for (int c = 0; c < W; ++c) cfma(t[c], cconj(u), v[c][i]);
+            }
+#pragma unroll
+            for (int i = kk + 1; i < NB; ++i) {
+                const double2 u = get(uoff(kk) + i);
+#pragma unroll
+                for (int c = 0; c < W; ++c) v[c][i] = csub(v[c][i], cmul(u, t[c]));
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < NB; ++i)
+#pragma unroll
+            for (int c = 0; c < W; ++c) stg[lane * G::STG + 2 * i + c] = v[c][i];
+        __syncwarp();
+        for (int x = lane; x < cnt * NB * W; x += 32) {
+            const int mat = x / (NB * W), r = x - mat * (NB * W), i = r / W, c = r - i * W;
+            if (c < nc) Vout[((size_t)(k0 + mat) * NB + i) * NB + c0 + c] = stg[mat * G::STG + r];
+        }
+    }
+}
+
+template <int NB>
+int launch_thread(const double2* M, double* w, double2* V, int64_t batch, int mode, cudaStream_t st) {
+    static std::once_flag once;
+    std::call_once(once, [] { raise_smem(k_eigh_thread<NB>); });
+    const unsigned grid = (unsigned)((batch + kThreadCta - 1) / kThreadCta);
+    k_eigh_thread<NB><<<grid, kThreadCta, ThreadGeo<NB>::kSmem, st>>>(M, w, V, batch, mode);
+    CPPHF_LAUNCH_CHECK("eigh (thread per matrix)");
+    return CPPHF_OK;
+}
+
 }  // namespace
 
 bool eigh_small_enabled(int64_t nb) { return nb >= 2 && nb <= 8; }
 
 int eigh_small(const double2* M, double* w, double2* V, int64_t batch, int64_t nb, int mode, cudaStream_t st) {
-    const int64_t threads = batch * (nb <= 2 ? 2 : (nb <= 4 ? 4 : 8));
-    const unsigned grid = (unsigned)((threads + kHqlThreads - 1) / kHqlThreads);
+    // A thread's chain takes 2.6 (nb = 2) to 55 us (nb = 8) however small the batch,
+    // and the batch takes little more until every scheduler has two warps; the
+    // groups' chains are shorter from nb = 5 on, but their throughput is a third.
+    // Measured (thread / group, us): nb = 4 10.6 / 10.7 at 1296 matrices, 13.7 / 28.3
+    // at 36864; nb = 6 23.5 / 22.4 at 4608, 23.6 / 25.6 at 6912, 32.7 / 114 at 36864;
+    // nb = 8 53.4 / 42.5 at 6912, 52.7 / 53.2 at 9216, 81.4 / 249 at 36864.
+    const int64_t least = nb <= 4 ? 0 : nb <= 6 ? 5632 : 9216;
+    if (batch >= least) {
+        switch (nb) {
+            case 2: return launch_thread<2>(M, w, V, batch, mode, st);
+            case 3: return launch_thread<3>(M, w, V, batch, mode, st);
+            case 4: return launch_thread<4>(M, w, V, batch, mode, st);
+            case 5: return launch_thread<5>(M, w, V, batch, mode, st);
+            case 6: return launch_thread<6>(M, w, V, batch, mode, st);
+            case 7: return launch_thread<7>(M, w, V, batch, mode, st);
+            case 8: return launch_thread<8>(M, w, V, batch, mode, st);
+            default: break;
+        }
+    }
+    const unsigned grid = (unsigned)((batch * kGroup + kHqlThreads - 1) / kHqlThreads);
     switch (nb) {
-        case 2: k_eigh_hql<2><<<grid, kHqlThreads, 0, st>>>(M, w, V, batch, mode); break;
-        case 3: k_eigh_hql<3><<<grid, kHqlThreads, 0, st>>>(M, w, V, batch, mode); break;
-        case 4: k_eigh_hql<4><<<grid, kHqlThreads, 0, st>>>(M, w, V, batch, mode); break;
         case 5: k_eigh_hql<5><<<grid, kHqlThreads, 0, st>>>(M, w, V, batch, mode); break;
         case 6: k_eigh_hql<6><<<grid, kHqlThreads, 0, st>>>(M, w, V, batch, mode); break;
         case 7: k_eigh_hql<7><<<grid, kHqlThreads, 0, st>>>(M, w, V, batch, mode); break;

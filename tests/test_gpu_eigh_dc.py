@@ -1,4 +1,4 @@
-"""GPU: the divide-and-conquer eigensolver (nb outside 2..8, and block structures) against LAPACK.
+"""GPU: the eigensolvers against LAPACK: divide and conquer (nb outside 2..8, block structures), QL (nb = 2..8).
 
 Sizes are the edges of its size classes (16, 24, 32, 48, 64, 80) and of its
 merge tree.  A backward stable solver has residual, orthogonality and
@@ -37,7 +37,7 @@ def matrices(nb, r):
         U = unitary(r, nb)
         out.append((U * lam) @ U.conj().T)
     D = np.diag(np.round(3 * r.normal(size=nb))).astype(complex)
-    out += [D, np.zeros((nb, nb), complex), D + 1e-17 * out[0], 1e-200 * out[0], 1e200 * out[0]]
+    out += [D, np.zeros((nb, nb), complex), D + 1e-17 * out[0], D + 1e-158 * out[0], 1e-200 * out[0], 1e200 * out[0]]
     out.append(2 * np.eye(nb) + np.eye(nb, k=1) + np.eye(nb, k=-1) + 0j)
     return np.array([0.5 * (M + M.conj().T) for M in out])
 
@@ -57,6 +57,21 @@ def test_against_lapack(native, nb):
     w, V = native.eigh_batched(M)
     check(M, w, V)
     for A, wk in zip(M, w):
+        wr = np.linalg.eigvalsh(A)
+        assert np.all(np.diff(wk) >= 0)
+        assert np.abs(wk - wr).max() <= 20 * nb * EPS * np.abs(wr).max()
+
+
+@pytest.mark.parametrize("batch", (1, 33, 9300))  # one thread, a partial warp, a batch past every rule
+@pytest.mark.parametrize("nb", range(2, 9))
+def test_small(native, nb, batch):
+    """nb = 2..8: a thread or eight lanes per matrix, by batch."""
+    M = matrices(nb, np.random.default_rng(nb))
+    M = np.concatenate([M] * (batch // len(M) + 1))[:batch]
+    w, V = native.eigh_batched(M)
+    n = min(batch, 64)
+    check(M[-n:], w[-n:], V[-n:])
+    for A, wk in zip(M[-n:], w[-n:]):
         wr = np.linalg.eigvalsh(A)
         assert np.all(np.diff(wk) >= 0)
         assert np.abs(wk - wr).max() <= 20 * nb * EPS * np.abs(wr).max()
