@@ -1,47 +1,72 @@
-// Chemical-potential solvers as one cooperative persistent kernel each
-// (cpp_hf utils.hpp:49-116).
+// Chemical-potential solvers as one persistent kernel each (cpp_hf utils.hpp:49-116).
 //
-// Every block owns a contiguous slice of the (nk*nb) eigenvalues.  Per round
-// a block reduces its slice (fixed tree) into partials, the grid meets at a
-// bounded barrier, every block sums all blocks' partials with the same fixed
-// tree and replays the reference's scalar update rule itself, so the whole grid
-// agrees on (lo, hi, mu).  The results are those of the reference's fixed
-// iteration counts (30 bisection steps by default, mu_maxiter Newton steps).
-// Bisection runs its first levels as exact multisection rounds, then finds
-// the root of N(mu) = n_e by Newton and replays the remaining levels against
-// it (a level whose midpoint lies within the rounding margin of the root is
-// counted exactly), which reproduces the bisection's decisions with a few
-// counts instead of one per level.  Newton stops early only once its state
-// (mu, lo, hi) repeats with period 1 or 2, when the state after the remaining
-// iterations is already known.
+// Every block owns a slice of the (nk*nb) eigenvalues.  Per round a block reduces
+// its slice (fixed tree), publishes its sums, takes everyone else's and adds all
+// of them with the same fixed tree, so the whole grid agrees on (lo, hi, mu) and
+// replays the reference's scalar update rule itself.  The results are those of the
+// reference's fixed iteration counts (30 bisection steps by default, mu_maxiter
+// Newton steps).  Bisection runs its first levels as exact multisection rounds,
+// then finds the root of N(mu) = n_e by Newton and replays the remaining levels
+// against it (a level whose midpoint lies within the rounding margin of the root is
+// counted exactly), which reproduces the bisection's decisions with a few counts
+// instead of one per level.  Newton stops early only once its state (mu, lo, hi)
+// repeats with period 1 or 2, when the state after the remaining iterations is
+// already known.
+//
+// A round is latency: two exponentials, two block trees and one exchange between
+// the blocks.  In the cooperative grid the exchange needs no barrier: each round
+// has slots of its own, cleared to a NaN pattern before the launch, a block stores
+// its sums into its slot and every block polls all slots until they hold numbers.
+// The sums are their own flags, so a round is one store and one L2 round trip
+// instead of a counter, a generation word, their fences and a second read.
+// Measured against that barrier (bisection / in-loop Newton, us): 294912
+// eigenvalues 78 / 57 -> 60 / 35, 82944 66 / 55 -> 54 / 40, 4608 103 / 57 -> 27 / 16.5
+// (one block -> one cluster).
 #include "common.cuh"
 #include "mu.cuh"
 
-#include <cstdlib>
 #include <mutex>
 
 namespace cpphf {
 
 namespace {
 
-constexpr int kMuThreads = 1024;
+// 512 threads: the shuffles of the two block trees are a third of a round, and
+// halve against 1024 (294912 eigenvalues: 71 -> 60 us bisection, 51 -> 35 in-loop)
+constexpr int kMuThreads = 512;
 constexpr int kMuMaxGrid = 1024;
-constexpr int kMuCache = 2;                           // eigenvalues a thread keeps in registers across rounds
-constexpr int64_t kMuOneBlockMax = 32768;             // eigenvalues handled by a single CTA
+constexpr int kMuCache = 4;                           // eigenvalues a thread keeps in registers across rounds
+// Forms by the number of eigenvalues, each an ordinary launch but the last.
+// Measured (bisection / in-loop Newton, us), one block against one cluster: 24.8 /
+// 14.5 and 22.8 / 16.5 at 1152 eigenvalues, 53 / 29 and 27 / 16.5 at 4608; one
+// cluster against the cooperative grid: 51 / 31 and 53 / 21 at 18432, 62 / 41 and
+// 47 / 34 at 36864, 118 / 78 and 55 / 29 at 73728.  Up to 2^16 the cluster is kept:
+// concurrent solves (a sweep on 16 streams) do not wait for a whole grid of SMs.
+constexpr int64_t kMuOneBlockMax = 1024;              // eigenvalues handled by a single CTA
 constexpr int kMuCluster = 8;                         // CTAs of the cluster form (portable cluster size)
-// eigenvalues handled by one cluster: up to 8 per thread and round; beyond
-// that the cooperative grid's extra SMs outweigh its software barriers
-constexpr int64_t kMuClusterMax = (int64_t)1 << 16;
+constexpr int64_t kMuClusterMax = (int64_t)1 << 16;   // eigenvalues handled by one cluster
 constexpr int kBisectLevels = 3;                      // bisection steps per grid barrier
 constexpr int kMuNV = (1 << kBisectLevels) - 1;       // midpoints evaluated per barrier
 constexpr double kMuWide = 64.0;                      // exact multisection while the bracket exceeds 64 T
 constexpr int kMuWarmMaxIter = 8;                     // Newton rounds from a warm start before the cold path
+constexpr int kMuSlots = 40;                          // slots of a call (rounds before they are cleared and reused)
+// barrier words, then slots of 16 bytes per block (fewer than kMuSlots of them on a grid above 205 blocks)
+constexpr size_t kMuWsBytes = 64 + 16 * (size_t)8 * kMuMaxGrid;
 constexpr int kMuRootMaxIter = 80;                    // safeguarded Newton rounds (bisection fallback)
 
 __device__ __forceinline__ double expit(double x) {
     if (x >= 0.0) return 1.0 / (1.0 + exp(-x));
     const double e = exp(x);
     return e / (1.0 + e);
+}
+
+// (p, p (1 - p)) of p = 1 / (1 + exp(-x)) from one exponential and one
+// reciprocal: as exact as expit (and p (1 - p) without its cancellation), in half
+// the instructions.  A single block keeps the reference's own expressions: small
+// solves that stop on a plateau depend on the last bits of N(mu).
+__device__ __forceinline__ double2 fermi(double x) {
+    const double e = exp(-fabs(x)), r = 1.0 / (1.0 + e), er = e * r;
+    return mk(x >= 0.0 ? r : er, er * r);
 }
 
 // Shortcut thresholds on the (approximate) logistic argument x: for x >= 37,
@@ -64,7 +89,8 @@ struct MuArgs {
     int maxiter;
     int mode;  // 0 bisection (utils.hpp:49-75), 1 in-loop newton (utils.hpp:79-116)
     double* mu_out;
-    double* part;     // [grid][2] min/max, then two [grid][kMuNV] partials buffers (by round parity)
+    double* slots;    // [nslots][grid] pairs: the rounds' published sums
+    int nslots;
     unsigned* sync;   // [0] count [1] gen [2] error
     unsigned* err;    // device error word (may be null)
     long long spin_limit;  // grid-barrier poll limit
@@ -87,69 +113,144 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Grid-wide synchronisation of the mu kernel.  CLUSTER = false: a cooperative
-// grid with the bounded software barrier; CLUSTER = true: one thread-block
-// cluster (kMuCluster CTAs) with the hardware cluster barrier.  In both, every
-// block sums all blocks' partials itself in the same fixed order after the
-// barrier (a few KB from L2; no block waits for a last arriver's reduction), so
-// the partials are double-buffered by round parity (a block may start writing
-// round r + 1 while another still reads round r).
+__device__ __forceinline__ double2 ld_slot(const double2* p) {
+    double2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_slot(double2* p, double2 v) {
+    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(v.x), "d"(v.y) : "memory");
+}
+// the pattern of an empty slot half; no arithmetic result has it
+__device__ __forceinline__ bool empty(double x) { return __double_as_longlong(x) == -1LL; }
+__device__ __forceinline__ double full(double x) { return empty(x) ? NAN : x; }
+
+// Sums (or maxima) over all eigenvalues, one round at a time.  CLUSTER = false: a
+// cooperative grid, or a single block; CLUSTER = true: one thread-block cluster
+// (kMuCluster CTAs) with the hardware cluster barrier and partials in global
+// memory, double-buffered by round parity.
 template <bool CLUSTER>
 struct MuSync {
     GridBarrier bar;
-    double* ctot;  // shared totals
-    double (*red)[32 * kMuNV];  // the kernel's block_sum scratch
-    __device__ void init(const MuArgs& a, double* sh, double (*scratch)[32 * kMuNV]) {
-        if (!CLUSTER) bar.init(a.sync, a.spin_limit, a.err);
-        ctot = sh;
+    double2* slots;  // [nslots][G]
+    int nslots, slot, phase, G;
+    double (*red)[32 * kMuNV];  // two trees' scratch, used alternately
+    int* failed;
+    unsigned* err;
+    long long limit;
+    __device__ void init(const MuArgs& a, double (*scratch)[32 * kMuNV], int* fail_flag) {
+        bar.init(a.sync, a.spin_limit, a.err);
+        slots = reinterpret_cast<double2*>(a.slots);
+        nslots = a.nslots;
+        slot = phase = 0;
+        G = gridDim.x;
         red = scratch;
+        failed = fail_flag;
+        err = a.err;
+        limit = a.spin_limit;
     }
-    __device__ bool all() {
-        if constexpr (CLUSTER) {
-            cluster_sync_all();
-            return true;
-        } else {
-            return bar.wait();
-        }
+    template <bool MAX>
+    static __device__ __forceinline__ double op(double a) {
+        return MAX ? warp_max(a) : warp_sum(a);
     }
-    // the partials buffer of a round
-    __device__ double* partials(double* part, int round) const {
-        return part + (size_t)(round & 1) * kMuNV * gridDim.x;
-    }
-    // every block's NV partials summed (fixed order); null if a wait gave up
-    template <int NV>
-    __device__ const double* reduce(const double* part, int G) {
-        if constexpr (CLUSTER) {
-            cluster_sync_all();
-        } else {
-            if (!bar.wait()) return nullptr;
-        }
-        // all threads load the partials at once (one L2 round trip), then the
-        // block's fixed tree: every block forms the same totals
-        double v[NV];
+    // fixed tree over the block; every thread gets the result
+    template <int NV, bool MAX>
+    __device__ __forceinline__ void tree(double (&v)[NV]) {
+        double* s = red[phase & 1];
+        ++phase;
+        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-        for (int j = 0; j < NV; ++j) v[j] = 0.0;
-        for (int b = threadIdx.x; b < G; b += blockDim.x) {
-#pragma unroll
-            for (int j = 0; j < NV; ++j) v[j] += __ldcg(&part[NV * b + j]);
-        }
-        block_sum<NV>(v, *red);
-        if (threadIdx.x == 0) {
-#pragma unroll
-            for (int j = 0; j < NV; ++j) ctot[j] = v[j];
+        for (int i = 0; i < NV; ++i) {
+            v[i] = op<MAX>(v[i]);
+            if (lane == 0) s[32 * i + wid] = v[i];
         }
         __syncthreads();
-        return ctot;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) v[i] = op<MAX>(lane < kMuThreads / 32 ? s[32 * i + lane] : (MAX ? -INFINITY : 0.0));
     }
-    __device__ double load(const double* t, int j) const { return t[j]; }
+    // all blocks' values combined, in every thread; false if a wait gave up
+    template <int NV, bool MAX = false>
+    __device__ bool reduce(double (&v)[NV]) {
+        tree<NV, MAX>(v);
+        if (G == 1) return true;
+        constexpr int NS = (NV + 1) / 2;
+        if constexpr (CLUSTER) {
+            // G = kMuCluster <= 32: every warp reads all partials
+            double2* b = slots + (size_t)(slot & 1) * 4 * G;
+            ++slot;
+            if (threadIdx.x == 0) {
+#pragma unroll
+                for (int u = 0; u < NS; ++u)
+                    __stcg(&b[u * G + blockIdx.x], mk(v[2 * u], 2 * u + 1 < NV ? v[2 * u + 1] : 0.0));
+            }
+            cluster_sync_all();
+            const int lane = threadIdx.x & 31;
+#pragma unroll
+            for (int u = 0; u < NS; ++u) {
+                const double2 x = lane < G ? __ldcg(&b[u * G + lane]) : mk(MAX ? (double)-INFINITY : 0.0, MAX ? (double)-INFINITY : 0.0);
+                v[2 * u] = op<MAX>(x.x);
+                if (2 * u + 1 < NV) v[2 * u + 1] = op<MAX>(x.y);
+            }
+            return true;
+        } else {
+            if (slot + NS > nslots && !recycle()) return false;
+            double2* b = slots + (size_t)slot * G;
+            slot += NS;
+            if (threadIdx.x == 0) {
+#pragma unroll
+                for (int u = 0; u < NS; ++u)
+                    st_slot(&b[u * G + blockIdx.x], mk(full(v[2 * u]), 2 * u + 1 < NV ? full(v[2 * u + 1]) : 0.0));
+            }
+#pragma unroll
+            for (int i = 0; i < NV; ++i) v[i] = MAX ? -INFINITY : 0.0;
+            bool ok = true;
+            for (int t = threadIdx.x; t < G && ok; t += kMuThreads) {
+#pragma unroll
+                for (int u = 0; u < NS; ++u) {
+                    double2 x = ld_slot(&b[u * G + t]);
+                    for (long long spins = 0; empty(x.x) || empty(x.y); x = ld_slot(&b[u * G + t])) {
+                        if (++spins > limit) {
+                            ok = false;
+                            break;
+                        }
+                    }
+                    v[2 * u] = MAX ? fmax(v[2 * u], x.x) : v[2 * u] + x.x;
+                    if (2 * u + 1 < NV) v[2 * u + 1] = MAX ? fmax(v[2 * u + 1], x.y) : v[2 * u + 1] + x.y;
+                }
+            }
+            if (!ok) {
+                *failed = 1;
+                if (err) atomicOr(err, kWaitErrBarrier);
+            }
+            tree<NV, MAX>(v);  // its barrier also orders the flag
+            return *failed == 0;
+        }
+    }
+    // every slot is used: meet, clear one's own, meet again
+    __device__ bool recycle() {
+        if (!bar.wait()) return false;
+        for (int i = threadIdx.x; i < nslots; i += kMuThreads)
+            slots[(size_t)i * G + blockIdx.x] = mk(__longlong_as_double(-1LL), __longlong_as_double(-1LL));
+        slot = 0;
+        return bar.wait();
+    }
 };
 
 template <bool CLUSTER>
 __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
-    __shared__ double red[32 * kMuNV];  // block_sum<kMuNV> scratch (32 doubles per value)
-    __shared__ double ctot_sh[kMuNV];
-    MuSync<CLUSTER> bar;
-    bar.init(a, ctot_sh, &red);
+    __shared__ double red[2][32 * kMuNV];
+    __shared__ int failed;
+    if (threadIdx.x == 0) {
+        failed = 0;  // ordered by the first tree's barrier
+        if (!CLUSTER && blockIdx.x == 0 && gridDim.x > 1) {
+            // barrier words (the launch filled them with the empty pattern): visible before
+            // this block's first sums, without which no block comes to use them
+            a.sync[0] = a.sync[1] = a.sync[2] = 0u;
+            __threadfence();
+        }
+    }
+    MuSync<CLUSTER> net;
+    net.init(a, red, &failed);
     const int G = gridDim.x;
     const unsigned nb = (unsigned)a.nb;
     const unsigned n = (unsigned)a.n;
@@ -157,9 +258,8 @@ __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
     const unsigned e0 = blockIdx.x * per;
     const unsigned e1 = min(n, e0 + per);
     // The thread's eigenvalues and weights (band-major), loaded once: with at
-    // most kMuCache of them per thread (the cooperative grid at the sizes the
-    // solvers run) they stay in registers for every round; otherwise every
-    // round reloads them.  Same elements, same order either way.
+    // most kMuCache of them per thread they stay in registers for every round;
+    // otherwise every round reloads them.  Same elements, same order either way.
     const bool cached = (per + blockDim.x - 1) / blockDim.x <= (unsigned)kMuCache;  // grid-uniform
     double cw[kMuCache], ce[kMuCache];
 #pragma unroll
@@ -182,56 +282,28 @@ __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
             }
         }
     };
+    auto give_up = [&]() {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *a.mu_out = NAN;
+    };
 
     // 1. global min / max of eps
-    double lmin = INFINITY, lmax = -INFINITY;
-    for (unsigned i = e0 + threadIdx.x; i < e1; i += blockDim.x) {
-        const double e = a.eps[i];
-        lmin = fmin(lmin, e);
-        lmax = fmax(lmax, e);
-    }
-    {
-        double v[2] = {-lmin, lmax};
-        // max-reduce through the sum scratch: use warp max then smem
-        v[0] = warp_max(v[0]);
-        v[1] = warp_max(v[1]);
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-        if (lane == 0) {
-            red[wid] = v[0];
-            red[32 + wid] = v[1];
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double m0 = -INFINITY, m1 = -INFINITY;
-            for (int i = 0; i < nw; ++i) {
-                m0 = fmax(m0, red[i]);
-                m1 = fmax(m1, red[32 + i]);
+    double ends[2] = {-INFINITY, -INFINITY};  // -min, max
+    if (cached) {
+#pragma unroll
+        for (int u = 0; u < kMuCache; ++u)
+            if (e0 + threadIdx.x + u * blockDim.x < e1) {
+                ends[0] = fmax(ends[0], -ce[u]);
+                ends[1] = fmax(ends[1], ce[u]);
             }
-            a.part[2 * blockIdx.x] = m0;
-            a.part[2 * blockIdx.x + 1] = m1;
+    } else {
+        for (unsigned i = e0 + threadIdx.x; i < e1; i += blockDim.x) {
+            const double e = a.eps[i];
+            ends[0] = fmax(ends[0], -e);
+            ends[1] = fmax(ends[1], e);
         }
     }
-    if (!bar.all()) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) *a.mu_out = NAN;
-        return;
-    }
-    // warp 0 reduces the block partials (fixed lane-strided order) and broadcasts
-    __shared__ double bc[2];
-    if (threadIdx.x < 32) {
-        double m0 = -INFINITY, m1 = -INFINITY;
-        for (int b = threadIdx.x; b < G; b += 32) {
-            m0 = fmax(m0, __ldcg(&a.part[2 * b]));
-            m1 = fmax(m1, __ldcg(&a.part[2 * b + 1]));
-        }
-        m0 = warp_max(m0);
-        m1 = warp_max(m1);
-        if (threadIdx.x == 0) {
-            bc[0] = -m0;
-            bc[1] = m1;
-        }
-    }
-    __syncthreads();
-    const double emin = bc[0], emax = bc[1];
+    if (!net.template reduce<2, true>(ends)) return give_up();
+    const double emin = -ends[0], emax = ends[1];
     const double Tj = fmax(a.T, 1.0e-12);
     double lo, hi, mu = 0.0;
     if (a.mode == 0) {
@@ -245,9 +317,6 @@ __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
     }
     const double Tfd = Tj + 1.0e-12;  // fermidirac_scalar(x, Tj) = expit(-x / (Tj + 1e-12))
     const double invTfd = 1.0 / Tfd, invTj = 1.0 / Tj;
-    double* part0 = a.part + 2 * G;  // two [G][kMuNV] partials buffers, by round parity
-    __shared__ double bc_tot[kMuNV];
-    int round = 0;
     if (a.mode == 0) {
         // Bisection (utils.hpp:49-75) in three phases.
         //  1. Exact multisection rounds while the bracket is wide: the counts at
@@ -300,42 +369,34 @@ __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
                         if (xa >= kFdOne)
                             v[j] += wk;
                         else if (xa > kFdZero)
-                            v[j] += wk * expit(-(e - mid[j]) / Tfd);
+                            v[j] += wk * (G == 1 ? expit(-(e - mid[j]) / Tfd) : fermi(xa).x);
                     }
                 }
             });
-            block_sum<kMuNV>(v, red);
-            double* part = bar.partials(part0, round);
-            if (threadIdx.x == 0) {
-#pragma unroll
-                for (int j = 0; j < kMuNV; ++j) __stcg(&part[kMuNV * blockIdx.x + j], v[j]);
-            }
-            const double* tot = bar.template reduce<kMuNV>(part, G);
-            if (!tot) {
+            if (!net.template reduce<kMuNV>(v)) {
                 ok = false;
                 return;
             }
-            if (threadIdx.x < kMuNV) bc_tot[threadIdx.x] = bar.load(tot, threadIdx.x);
-            __syncthreads();
             int node = 0;
             for (int l = 0; l < L; ++l) {
-                double m = mid[0];
+                double m = mid[0], N = v[0];
 #pragma unroll
                 for (int j = 1; j < kMuNV; ++j)
-                    if (j == node) m = mid[j];
-                if (bc_tot[node] > a.target) {
+                    if (j == node) {
+                        m = mid[j];
+                        N = v[j];
+                    }
+                if (N > a.target) {
                     hi = m;
-                    Nhi = bc_tot[node];
+                    Nhi = N;
                     node = 2 * node + 1;
                 } else {
                     lo = m;
-                    Nlo = bc_tot[node];
+                    Nlo = N;
                     node = 2 * node + 2;
                 }
             }
-            __syncthreads();
             it += L;
-            ++round;
         };
         // count N and slope Z = dN/dmu at one mu (one grid round)
         auto count_round = [&](double m, double& N, double& Z) {
@@ -345,28 +406,23 @@ __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
                 if (xa >= kFdOne) {
                     v[0] += wk;
                 } else if (xa > kFdZero) {
-                    const double pf = expit(-(e - m) / Tfd);
-                    v[0] += wk * pf;
-                    v[1] += wk * pf * (1.0 - pf) * invTfd;
+                    if (G == 1) {
+                        const double pf = expit(-(e - m) / Tfd);
+                        v[0] += wk * pf;
+                        v[1] += wk * pf * (1.0 - pf) * invTfd;
+                    } else {
+                        const double2 f = fermi(xa);
+                        v[0] += wk * f.x;
+                        v[1] += wk * f.y * invTfd;
+                    }
                 }
             });
-            block_sum<2>(v, red);
-            double* part = bar.partials(part0, round);
-            if (threadIdx.x == 0) {
-                __stcg(&part[2 * blockIdx.x], v[0]);
-                __stcg(&part[2 * blockIdx.x + 1], v[1]);
-            }
-            const double* tot = bar.template reduce<2>(part, G);
-            ++round;
-            if (!tot) {
+            if (!net.template reduce<2>(v)) {
                 ok = false;
                 return;
             }
-            if (threadIdx.x < 2) bc_tot[threadIdx.x] = bar.load(tot, threadIdx.x);
-            __syncthreads();
-            N = bc_tot[0];
-            Z = bc_tot[1];
-            __syncthreads();
+            N = v[0];
+            Z = v[1];
         };
         // safeguarded Newton for the root of N(mu) = target inside [ra, rb]
         struct Root {
@@ -444,10 +500,7 @@ __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
                     while (ok && it < a.maxiter) msec_round();
             }
         }
-        if (!ok) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) *a.mu_out = NAN;
-            return;
-        }
+        if (!ok) return give_up();
     } else {
         // Newton in a bracket.  The update is a deterministic function of the
         // state (mu, lo, hi); once the state repeats with period 1 or 2 the
@@ -463,26 +516,19 @@ __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
                 if (xa >= kFdOne) {
                     v[0] += wk;
                 } else if (xa > kFdZero) {
-                    const double p = expit((mu - e) / Tj);
-                    v[0] += wk * p;
-                    v[1] += wk * p * (1.0 - p) / Tj;
+                    if (G == 1) {
+                        const double p = expit((mu - e) / Tj);
+                        v[0] += wk * p;
+                        v[1] += wk * p * (1.0 - p) / Tj;
+                    } else {
+                        const double2 f = fermi(xa);
+                        v[0] += wk * f.x;
+                        v[1] += wk * f.y * invTj;
+                    }
                 }
             });
-            block_sum<2>(v, red);
-            double* part = bar.partials(part0, it);
-            if (threadIdx.x == 0) {
-                __stcg(&part[2 * blockIdx.x], v[0]);
-                __stcg(&part[2 * blockIdx.x + 1], v[1]);
-            }
-            const double* tot = bar.template reduce<2>(part, G);
-            if (!tot) {
-                if (blockIdx.x == 0 && threadIdx.x == 0) *a.mu_out = NAN;
-                return;
-            }
-            if (threadIdx.x < 2) bc_tot[threadIdx.x] = bar.load(tot, threadIdx.x);
-            __syncthreads();
-            const double N = bc_tot[0], Z = bc_tot[1];
-            __syncthreads();
+            if (!net.template reduce<2>(v)) return give_up();
+            const double N = v[0], Z = v[1];
             const double mu0 = mu, lo0 = lo, hi0 = hi;
             const double g = N - a.target;
             if (g < 0.0) lo = mu;
@@ -529,14 +575,12 @@ int max_coop_grid() {
 // launches.  Every GPU that loads the library holds it until the process
 // exits; every call shares it.
 // ---------------------------------------------------------------------------
-constexpr size_t kMuNoAllocScratchBytes = 64 + sizeof(double) * ((2 + 2 * kMuNV) * (size_t)kMuMaxGrid + 2 * kMuNV);
+constexpr size_t kMuNoAllocScratchBytes = kMuWsBytes;
 static __device__ __align__(256) unsigned char g_mu_noalloc_scratch[kMuNoAllocScratchBytes];
 
 }  // namespace
 
-size_t mu_workspace_bytes(int64_t, int64_t) {
-    return 64 + sizeof(double) * ((2 + 2 * kMuNV) * (size_t)kMuMaxGrid + 2 * kMuNV);
-}
+size_t mu_workspace_bytes(int64_t, int64_t) { return kMuWsBytes; }
 
 int mu_solve(const double* eps, const double* w, int64_t nk, int64_t nb, double target,
              const double* mu0, double T, int maxiter, int mode, double* mu_out, void* ws,
@@ -547,7 +591,7 @@ int mu_solve(const double* eps, const double* w, int64_t nk, int64_t nb, double 
     if (mode == 1 && !mu0) return fail(CPPHF_ERR_INVALID, "mu: null warm start");
     if (!ws || wsb < mu_workspace_bytes(nk, nb)) return fail(CPPHF_ERR_INVALID, "mu: workspace too small");
     const int64_t n = nk * nb;
-    int grid = (int)std::min<int64_t>(max_coop_grid(), (n + kMuThreads - 1) / kMuThreads);
+    int grid = (int)std::min<int64_t>(max_coop_grid(), (n + kMuThreads * kMuCache / 2 - 1) / (kMuThreads * kMuCache / 2));
     if (grid < 1) grid = 1;
     // small problems: one CTA does it all (its barriers are block-local), launched
     // as an ordinary kernel so that solves on other streams keep running beside it
@@ -567,8 +611,8 @@ int mu_solve(const double* eps, const double* w, int64_t nk, int64_t nb, double 
     a.err = wait_error_word();
     if (!a.err) return CPPHF_ERR_CUDA;
     a.spin_limit = barrier_spin_limit();
-    a.part = reinterpret_cast<double*>(static_cast<unsigned char*>(ws) + 64);
-    CPPHF_CUDA(cudaMemsetAsync(ws, 0, 64, st));
+    a.slots = reinterpret_cast<double*>(static_cast<unsigned char*>(ws) + 64);
+    a.nslots = 0;
     if (grid == 1) {
         k_mu<false><<<1, kMuThreads, 0, st>>>(a);
         CPPHF_LAUNCH_CHECK("mu (one block)");
@@ -592,6 +636,8 @@ int mu_solve(const double* eps, const double* w, int64_t nk, int64_t nb, double 
         CPPHF_CUDA(cudaLaunchKernelEx(&cfg, k_mu<true>, a));
         return CPPHF_OK;
     }
+    a.nslots = (int)std::min<int64_t>(kMuSlots, (int64_t)(kMuWsBytes - 64) / 16 / grid);
+    CPPHF_CUDA(cudaMemsetAsync(ws, 0xFF, 64 + 16 * (size_t)a.nslots * grid, st));
     void* args[] = {&a};
     CPPHF_CUDA(cudaLaunchCooperativeKernel((const void*)k_mu<false>, dim3(grid), dim3(kMuThreads), args, 0, st));
     return CPPHF_OK;
