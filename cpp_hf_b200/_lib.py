@@ -120,6 +120,7 @@ _SIGS = {
     "cpphf_build_fock_workspace_bytes": (sz, [C.POINTER(Kernel)]),
     "cpphf_kernel_packed_bytes": (sz, [C.POINTER(Kernel)]),
     "cpphf_kernel_pack": (C.c_int, [C.POINTER(Kernel), vp, vp, vp]),
+    "cpphf_vr_hermitian_deviation": (C.c_int, [vp, i64, i64, i64, vp, vp]),
     "cpphf_build_fock": (C.c_int, [C.POINTER(Kernel), vp, vp, vp, vp, vp, vp, vp, sz, vp]),
     "cpphf_cayley_spectral_setup": (C.c_int, [vp, vp, vp, i64, i64, vp]),
     "cpphf_cayley_unitary": (C.c_int, [vp, vp, f64, vp, i64, i64, vp]),

@@ -272,15 +272,11 @@ def _vr_hermitian(VR_t):
     R -> -R is the index map j -> (-j) mod n on both mesh axes; for a scalar VR
     (V real) the condition reads VR(R) == conj VR(-R).  Runs on the device.
     """
-    n0, n1 = VR_t.shape[0], VR_t.shape[1]
-    i0 = (-torch.arange(n0, device=VR_t.device)) % n0
-    i1 = (-torch.arange(n1, device=VR_t.device)) % n1
-    neg = VR_t.index_select(0, i0).index_select(1, i1)
-    scale = float(VR_t.abs().max())
-    if scale == 0.0:
-        return True
-    dev = float((VR_t.transpose(-1, -2) - neg.conj()).abs().max())
-    return dev <= 1e-12 * scale
+    out = torch.empty(2, dtype=torch.float64, device=VR_t.device)
+    check(_lib_handle().cpphf_vr_hermitian_deviation(_ptr(VR_t), VR_t.shape[0], VR_t.shape[1], VR_t.shape[2],
+                                                     _ptr(out), _stream()), "vr_hermitian_deviation")
+    scale, dev = out.tolist()
+    return scale == 0.0 or dev <= 1e-12 * scale
 
 
 class _DeviceKernel:
@@ -306,16 +302,20 @@ class _DeviceKernel:
             if tuple(refP.shape) != (nk1, nk2, nb, nb):
                 raise ValueError("refP must match h shape when has_refP is true")
         w2d = _to_dev(args["w2d"], "f").reshape(-1)
-        HH = _to_dev(args["HH"], "f").reshape(-1)
+        # arrays that the kernel does not use stay on the host (a small upload costs 12 us)
+        HH = args["HH"]
+        HH = _to_dev(HH, "f").reshape(-1) if args["include_hartree"] else None
         cg_host = np.asarray(args["contact_g"].cpu() if _is_torch(args["contact_g"]) else args["contact_g"],
                              dtype=np.float64)
         if cg_host.ndim != 1:
             raise ValueError("contact_g must be 1-D")
         n_contact = cg_host.shape[0]
         has_contact = bool(np.any(cg_host != 0.0)) or n_contact > 1
-        cg = _to_dev(cg_host, "f")
-        cOi = _to_dev(args["contact_Oi"], "c")
-        cOj = _to_dev(args["contact_Oj"], "c")
+        cOi, cOj = args["contact_Oi"], args["contact_Oj"]
+        if has_contact:
+            cg, cOi, cOj = _to_dev(cg_host, "f"), _to_dev(cOi, "c"), _to_dev(cOj, "c")
+        else:
+            cg = cOi = cOj = None
         self.sl = None
         if args.get("superlattice_fock_active", False) or args.get("superlattice_hartree_active", False):
             self.sl = _superlattice_struct(args, nb)
@@ -336,8 +336,8 @@ class _DeviceKernel:
         K.weight_sum = float(args["weight_sum"])
         K.h, K.VR = h.data_ptr(), VR.data_ptr()
         K.refP = refP.data_ptr() if refP is not None else None
-        K.w2d, K.HH = w2d.data_ptr(), HH.data_ptr()
-        K.contact_g, K.contact_Oi, K.contact_Oj = cg.data_ptr(), cOi.data_ptr(), cOj.data_ptr()
+        K.w2d = w2d.data_ptr()
+        K.HH, K.contact_g, K.contact_Oi, K.contact_Oj = (None if t is None else t.data_ptr() for t in (HH, cg, cOi, cOj))
         if self.sl is not None:
             K.sl = C.pointer(self.sl[0])
         K.hermitian_packing = 0

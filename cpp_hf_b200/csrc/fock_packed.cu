@@ -79,6 +79,35 @@ __global__ void k_pack_fields(const double2* __restrict__ VR, int dv, const doub
     }
 }
 
+// out[0] = max |VR|, out[1] = max |VR_ba(R) - conj VR_ab(-R)| (R -> -R is j -> -j
+// mod n on both axes), as the bit patterns of non-negative doubles, whose integer
+// order is theirs (a NaN is above all).
+__device__ __forceinline__ unsigned long long bits_abs(double2 v) {
+    return (unsigned long long)__double_as_longlong(hypot(v.x, v.y)) & 0x7fffffffffffffffull;
+}
+__global__ void k_vr_hermitian(const double2* __restrict__ VR, int n0, int n1, int dv, unsigned long long* out) {
+    const int dv2 = dv * dv;
+    const int64_t n = (int64_t)n0 * n1 * dv2;
+    unsigned long long big = 0, dev = 0;
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t q = e / dv2;
+        const int r = (int)(e - q * dv2), a = r / dv, b = r - a * dv;
+        const int i = (int)(q / n1), j = (int)(q - (int64_t)i * n1);
+        const int64_t neg = (int64_t)(i ? n0 - i : 0) * n1 + (j ? n1 - j : 0);
+        const double2 x = VR[e], y = VR[neg * dv2 + b * dv + a];
+        big = max(big, bits_abs(x));
+        dev = max(dev, bits_abs(mk(y.x - x.x, y.y + x.y)));
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        big = max(big, __shfl_xor_sync(0xffffffffu, big, o));
+        dev = max(dev, __shfl_xor_sync(0xffffffffu, dev, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        if (big) atomicMax(&out[0], big);
+        if (dev) atomicMax(&out[1], dev);
+    }
+}
+
 // One tensor map per row-segment length L = 1..nb over a (n0, n1, nb*nb)
 // complex128 field viewed as {2 nb^2 doubles, n1, n0}: box {2L, N, 1}.
 struct SegMaps {
@@ -679,6 +708,20 @@ int build_fock_packed(const cpphf_kernel* K, const double2* P, double2* Sigma, d
 }  // namespace cpphf
 
 extern "C" {
+
+int cpphf_vr_hermitian_deviation(const void* VR, int64_t nk1, int64_t nk2, int64_t dv, double* out, void* stream) {
+    if (!VR || !out || nk1 < 1 || nk2 < 1 || dv < 1 || nk1 > 65535 || nk2 > 65535 || dv > 4096)
+        return cpphf::fail(CPPHF_ERR_INVALID, "vr_hermitian_deviation: bad arguments");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    CPPHF_CUDA(cudaMemsetAsync(out, 0, 2 * sizeof(double), st));
+    const int64_t n = nk1 * nk2 * dv * dv;
+    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)cpphf::num_sms() * 8));
+    cpphf::k_vr_hermitian<<<grid, 256, 0, st>>>(static_cast<const double2*>(VR), (int)nk1, (int)nk2, (int)dv,
+                                                reinterpret_cast<unsigned long long*>(out));
+    CPPHF_LAUNCH_CHECK("VR Hermitian check");
+    return CPPHF_OK;
+}
+
 
 size_t cpphf_kernel_packed_bytes(const cpphf_kernel* K) { return cpphf::packed_field_bytes(K); }
 

@@ -397,36 +397,74 @@ int block_problem_invariant(const cpphf_kernel* K, bool project, const BlockSpec
     return CPPHF_OK;
 }
 
-// The legacy default stream cannot be captured: a solve called on it runs on
-// its own non-blocking stream, ordered after the caller's stream on entry and
-// before it on exit.  A solve on any other stream runs (and is captured) on
-// that stream directly.  `capturable` is false when the private stream could
-// not be created; the solve then runs on the caller's stream without graphs.
-struct SolveStream {
-    cudaStream_t user = nullptr, s = nullptr;
+// The private stream of a host thread on one device, with the event that orders it
+// with the caller's stream: made by the thread's first solve on the legacy default
+// stream and kept until the thread ends (creating and destroying a stream takes
+// 110 us, as much as an iteration of a small solve).
+struct ThreadStream {
+    cudaStream_t s = nullptr;
     cudaEvent_t ev = nullptr;
+    bool tried = false;
+    ~ThreadStream() {
+        if (s) cudaStreamDestroy(s);
+        if (ev) cudaEventDestroy(ev);
+    }
+};
+constexpr int kMaxDevices = 64;
+
+ThreadStream* thread_stream() {
+    thread_local ThreadStream per_device[kMaxDevices];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    ThreadStream& t = per_device[dev];
+    if (!t.tried) {
+        t.tried = true;
+        if (cudaEventCreateWithFlags(&t.ev, cudaEventDisableTiming) != cudaSuccess ||
+            cudaStreamCreateWithFlags(&t.s, cudaStreamNonBlocking) != cudaSuccess) {
+            (void)cudaGetLastError();
+            t.s = nullptr;
+        }
+    }
+    return t.s ? &t : nullptr;
+}
+
+// The legacy default stream cannot be captured: a solve called on it runs on its
+// thread's own non-blocking stream, ordered after the caller's stream on entry and
+// before it on exit.  A solve on any other stream runs (and is captured) on that
+// stream directly.  `capturable` is false when there is no private stream; the
+// solve then runs on the caller's stream without graphs.
+struct SolveStream {
+    cudaStream_t user = nullptr;
+    ThreadStream* own = nullptr;
     bool capturable = true;
     explicit SolveStream(cudaStream_t u) : user(u) {
         if (u != nullptr && u != cudaStreamLegacy) return;
-        if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess ||
-            cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventRecord(ev, user) != cudaSuccess || cudaStreamWaitEvent(s, ev, 0) != cudaSuccess) {
+        own = thread_stream();
+        if (own && (cudaEventRecord(own->ev, user) != cudaSuccess || cudaStreamWaitEvent(own->s, own->ev, 0) != cudaSuccess)) {
             (void)cudaGetLastError();
-            if (s) cudaStreamDestroy(s);
-            s = nullptr;
-            capturable = false;
+            own = nullptr;
         }
+        capturable = own != nullptr;
     }
     ~SolveStream() {
-        if (s) {
-            cudaEventRecord(ev, s);
-            cudaStreamWaitEvent(user, ev, 0);
-            cudaStreamDestroy(s);
+        if (own) {
+            cudaEventRecord(own->ev, own->s);
+            cudaStreamWaitEvent(user, own->ev, 0);
         }
-        if (ev) cudaEventDestroy(ev);
     }
-    cudaStream_t stream() const { return s ? s : user; }
+    cudaStream_t stream() const { return own ? own->s : user; }
 };
+
+// Iterations launched kernel by kernel before one is captured.  A capture costs
+// about 340 us for the two parities of a DM iteration and 180 us for an SCF
+// iteration, and saves 25 to 35 us on each iteration after it, so a solve that is
+// done by then is better off without (measured on 48 x 48, nb = 2, and on
+// 192 x 192, nb = 8).
+constexpr int64_t kGraphAfterDm = 12;
+constexpr int64_t kGraphAfterScf = 8;
 
 // One DM iteration as an instantiated graph, per (buffer parity, precision).
 struct IterGraphs {
@@ -613,9 +651,9 @@ int solve_dm(const cpphf_kernel* K, const cpphf_dm_config* cfg, const double2* P
         const int cur = (int)(k & 1), prv = cur ^ 1;
         IterGraphs& gr = graphs;
         const int lw = low ? 1 : 0;
-        if (use_graphs && !gr.exec[cur][lw] && !gr.failed[cur][lw] && k - k0 >= 1) {
-            // capture this parity and precision once (after an eager iteration
-            // has set every kernel attribute); a failed capture runs eagerly
+        if (use_graphs && !gr.exec[cur][lw] && !gr.failed[cur][lw] && k - k0 >= kGraphAfterDm) {
+            // capture this parity and precision once (the iterations before have
+            // set every kernel attribute); a failed capture runs eagerly
             cudaGraph_t g = nullptr;
             if (cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
                 gr.failed[cur][lw] = true;
@@ -900,6 +938,7 @@ int solve_scf(const cpphf_kernel* K, const cpphf_scf_config* cfg, const double2*
     const bool fuse_mix = scf_graphs && dm_small_supported(nb);
     IterGraphs sgr;
     bool pending_mix = false;
+    int64_t k_switch = 0;  // first iteration in the current precision
     while (k < max_iter && !converged) {
         double2* comm_out = acc == 1 ? Rh + (size_t)hhead * nel : nullptr;
         auto body = [&]() -> int {
@@ -916,7 +955,7 @@ int solve_scf(const cpphf_kernel* K, const cpphf_scf_config* cfg, const double2*
         };
         const int lw = low ? 1 : 0;
         bool replayed = false;
-        if (scf_graphs && (pending_mix || fuse_mix) && d_hermitian) {
+        if (scf_graphs && (pending_mix || fuse_mix) && d_hermitian && k - k_switch >= kGraphAfterScf) {
             if (!sgr.exec[0][lw] && !sgr.failed[0][lw]) {
                 cudaGraph_t g = nullptr;
                 if (cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
@@ -972,6 +1011,7 @@ int solve_scf(const cpphf_kernel* K, const cpphf_scf_config* cfg, const double2*
             // switch: mix as usual; the next build runs in complex128
             low = false;
             converged = false;
+            k_switch = k + 1;
         }
         if (Dpre && !converged) CPPHF_CUDA(cudaMemcpyAsync(Dpre, D, fbytes, cudaMemcpyDeviceToDevice, st));
         d_hermitian = true;

@@ -203,6 +203,10 @@ typedef struct cpphf_kernel {
  * cpphf_build_fock accepts Sigma == NULL (no Sigma written).  No counterpart in
  * the reference for orbital V. */
 size_t cpphf_kernel_packed_bytes(const cpphf_kernel* K);
+/* out[0] = max |VR| and out[1] = max |VR_ba(R) - conj VR_ab(-R)| (two device
+ * doubles) of a complex128 (nk1, nk2, dv, dv) VR: V(q) is Hermitian at every q
+ * when the second vanishes. */
+int cpphf_vr_hermitian_deviation(const void* VR, int64_t nk1, int64_t nk2, int64_t dv, double* out, void* stream);
 /* VR_packed (may be NULL; needs dv == nb) and h_packed (may be NULL) of K. */
 int cpphf_kernel_pack(const cpphf_kernel* K, void* VR_packed, void* h_packed, void* stream);
 
