@@ -24,12 +24,15 @@
 //     unlike the n^2 dependent rotations of QL.
 //  3. The reflectors are applied to the eigenvectors, stored by ascending
 //     eigenvalue (stable) or, with block sizes, block by block.
-// What bounds it: the latency of the n reduction steps (two barriers, a square
-// root and a division each; half of the kernel at nb = 64), then the secular
-// iterations.  Measured against the cyclic Jacobi kernel it replaces (Hermitian
-// matrices with normal entries): 5184 of nb = 64 6.46 ms (84.7), 5184 of nb = 48
-// 3.31 (25.6), 2304 of nb = 32 0.47 (3.28), 9216 of nb = 24 1.07 (7.6), of
-// nb = 16 0.44 (1.29), of nb = 10 0.36 (0.48), 1296 of nb = 80 4.36 (39.2).
+// What bounds it: the latency of the n reduction steps (three barriers, two square
+// roots and a division each) and of the secular iterations, at two CTAs per SM for
+// nb = 64.  Measured against the cyclic Jacobi kernel it replaces (Hermitian
+// matrices with normal entries): 5184 of nb = 64 5.25 ms (84.7), 5184 of nb = 48
+// 2.72 (25.6), 2304 of nb = 32 0.44 (3.28), 9216 of nb = 24 1.05 (7.6), of
+// nb = 16 0.44 (1.29), of nb = 10 0.37 (0.48), 1296 of nb = 80 3.20 (39.2).  Walking
+// column k in its own four threads instead of taking row k from all columns, and
+// loading the operands of one row at a time, took 6.46 ms at nb = 64; unrolling the
+// loop over k / 4 (row blocks gone at compile time) 6.6 ms, for the code it makes.
 #include "common.cuh"
 #include "eigh.cuh"
 
@@ -63,11 +66,12 @@ template <int NE>
 struct DcSmem {
     static constexpr int NR = DcGeo<NE>::NR, LD = DcGeo<NE>::LD;
     double2 U[NR * (NR - 1) / 2];
-    double2 ub[2][NR], pb[2][NR], sub[NR];
+    double2 xb[2][NR], wb[NR], sub[NR];
     double Q[NR * LD], S[NR * LD];
     double beta[NR], d[NR], e[NR], z[NR], ds[NR], zs[NR], dk[NR], zk[NR], mu[NR], zh[NR], rc[NR], rs[NR];
-    double red[2][DcGeo<NE>::NT / 32];
-    int perm[NR], nd[NR], df[NR], org[NR], ra[NR], rb[NR], nrot[NR];
+    double red[2][DcGeo<NE>::NT / 32], red2[DcGeo<NE>::NT / 32], akk;
+    double2 s1;  // (A x)_{k+1}
+    int perm[NR], nd[NR], pc[NR], df[NR], org[NR], ra[NR], rb[NR], nrot[NR];
 };
 
 __device__ __forceinline__ double quad_sum(double v) {
@@ -83,6 +87,20 @@ __device__ __forceinline__ int quad_sum(int v) {
 __device__ __forceinline__ double quad_max(double v) {
     v = fmax(v, __shfl_xor_sync(0xffffffffu, v, 1));
     return fmax(v, __shfl_xor_sync(0xffffffffu, v, 2));
+}
+
+// a[i] for a CTA-uniform i: a jump instead of NE selects
+template <int NE>
+__device__ __forceinline__ double2 pick(const double2 (&a)[NE], int i) {
+    double2 v = a[NE - 1];
+    switch (i) {
+#define X(I) \
+    case I: v = a[I < NE ? I : 0]; break;
+        X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) X(17) X(18) X(19)
+#undef X
+        default: break;
+    }
+    return v;
 }
 
 // Root r of 1 + rho sum_i z_i^2 / (d_i - x), d ascending, as (pole, offset).
@@ -175,6 +193,7 @@ __global__ void __launch_bounds__(DcGeo<NE>::NT, DcGeo<NE>::BLOCKS)
     k_eigh_dc(const double2* __restrict__ M, double* __restrict__ w, double2* __restrict__ Vout, int n, int mode,
               const BlockSpec bs) {
     constexpr int LD = DcGeo<NE>::LD, NR = DcGeo<NE>::NR, NW = DcGeo<NE>::NT / 32;
+    constexpr int RG = NE % 4 == 0 ? 4 : 3;  // row blocks whose operands are loaded together
     extern __shared__ __align__(16) unsigned char smem_raw[];
     DcSmem<NE>& s = *reinterpret_cast<DcSmem<NE>*>(smem_raw);
     const int tid = threadIdx.x, q = tid & 3, j = tid >> 2, warp = tid >> 5, lane = tid & 31;
@@ -212,90 +231,136 @@ __global__ void __launch_bounds__(DcGeo<NE>::NT, DcGeo<NE>::BLOCKS)
     for (int t = 0; t < NW; ++t) amax = fmax(amax, s.red[0][t]);
     int ex = 0;
     if (amax > 0.0) frexp(amax, &ex);
+    const double sc0 = ldexp(1.0, -(ex / 2)), sc1 = ldexp(1.0, -(ex - ex / 2));
 #pragma unroll
-    for (int ii = 0; ii < NE; ++ii) a[ii] = mk(ldexp(a[ii].x, -ex), ldexp(a[ii].y, -ex));
+    for (int ii = 0; ii < NE; ++ii) {
+        // 2^-ex in two factors: it may itself be out of range
+        a[ii] = mk(a[ii].x * sc0 * sc1, a[ii].y * sc0 * sc1);
+    }
+    for (int t = tid; t < NR; t += blockDim.x) s.xb[0][t] = s.xb[1][t] = s.wb[t] = mk(0.0, 0.0);
     __syncthreads();
 
     // ---- 1. reduction ----
+    // A is Hermitian, so column k is the conjugate of row k, one element of it in a
+    // thread of every column: x = A[k+1:, k] and its norm need no thread to walk a
+    // column.  The product A x runs on the raw x while the first warp forms the
+    // reflector u = x + c e_{k+1}; A u = A x + c A[:, k+1] and u^H A u follow from
+    // the sums.
     for (int k = 0; k + 2 < n; ++k) {
-        const int b = k & 1;
-        double2* u = s.ub[b];
-        double2* p = s.pb[b];
-        if (j == k) {
-            const unsigned quad = 0xfu << (lane & 28);
-            double xn2 = 0.0;
-            double2 x0 = mk(0.0, 0.0);
-#pragma unroll
-            for (int ii = 0; ii < NE; ++ii) {
-                const int i = 4 * ii + q;
-                if (i > k) xn2 += a[ii].x * a[ii].x + a[ii].y * a[ii].y;
-                if (i == k + 1) x0 = a[ii];
-                if (i == k) s.d[k] = a[ii].x;
-            }
-            xn2 += __shfl_xor_sync(quad, xn2, 1);
-            xn2 += __shfl_xor_sync(quad, xn2, 2);
-            const int src = (lane & 28) + ((k + 1) & 3);
-            x0 = mk(__shfl_sync(quad, x0.x, src), __shfl_sync(quad, x0.y, src));
-            const double ax0 = modulus(x0), xn = sqrt(xn2);
-            const bool some = xn2 > kTinyNorm2;
-            const double2 ph = ax0 > 0.0 ? mk(x0.x / ax0, x0.y / ax0) : mk(1.0, 0.0);
-            double2* Uk = s.U + (size_t)k * (n - 1) - (size_t)k * (k - 1) / 2 - (k + 1);
-#pragma unroll
-            for (int ii = 0; ii < NE; ++ii) {
-                const int i = 4 * ii + q;
-                if (i > k && i < n) {
-                    const double2 ui = i == k + 1 ? mk(x0.x + ph.x * xn, x0.y + ph.y * xn) : a[ii];
-                    u[i] = ui;
-                    Uk[i] = ui;
+        const int kb = k >> 2, q2 = k & 3;
+        const double2 arow = pick<NE>(a, kb), ay = pick<NE>(a, (k + 1) >> 2);  // rows k and k + 1, where q has them
+        double2* x = s.xb[k & 1];
+        double2 xj = mk(0.0, 0.0);
+        const bool col = j > k && j < n;
+        if (warp * 8 + 7 >= k) {
+            double v = 0.0;
+            if (q == q2) {
+                if (col) {
+                    xj = cconj(arow);
+                    x[j] = xj;
+                    v = xj.x * xj.x + xj.y * xj.y;
+                } else if (j == k) {
+                    s.d[k] = arow.x;
                 }
             }
-            if (q == 0) {
-                s.beta[k] = some ? 1.0 / (xn * (xn + ax0)) : 0.0;
-                s.sub[k] = some ? mk(-ph.x * xn, -ph.y * xn) : x0;
+            v += __shfl_xor_sync(0xffffffffu, v, 4);
+            v += __shfl_xor_sync(0xffffffffu, v, 8);
+            v += __shfl_xor_sync(0xffffffffu, v, 16);
+            if (lane == q2) s.red[k & 1][warp] = v;
+        } else if (lane == 0) {
+            s.red[k & 1][warp] = 0.0;
+        }
+        __syncthreads();
+        // the reflector: u = x + c e_{k+1}, beta, and the new subdiagonal
+        if (tid == 0) {
+            double xn2 = 0.0;
+#pragma unroll
+            for (int t = 0; t < NW; ++t) xn2 += s.red[k & 1][t];
+            const double2 x0 = x[k + 1];
+            const double ax0 = modulus(x0), xn = sqrt(xn2);
+            const bool some = xn2 > kTinyNorm2;
+            const double iax = ax0 > 0.0 ? 1.0 / ax0 : 0.0;
+            const double2 ph = ax0 > 0.0 ? mk(x0.x * iax, x0.y * iax) : mk(1.0, 0.0);
+            s.beta[k] = some ? 1.0 / (xn * (xn + ax0)) : 0.0;
+            s.sub[k] = some ? mk(-ph.x * xn, -ph.y * xn) : x0;
+        }
+        double2 sj = mk(0.0, 0.0), yj = mk(0.0, 0.0);
+        if (warp * 8 + 7 > k) {
+            // (A x)_j over the rows below k (x is zero beyond n) and A[k+1, j]
+            double2 p0 = mk(0.0, 0.0), p1 = mk(0.0, 0.0);
+#pragma unroll
+            for (int g = 0; g < NE; g += RG)
+                if (g + RG > kb) {
+                    double2 xi[RG];
+#pragma unroll
+                    for (int h = 0; h < RG; ++h) {
+                        xi[h] = x[4 * (g + h) + q];
+                        if (4 * (g + h) + q <= k) xi[h] = mk(0.0, 0.0);
+                    }
+#pragma unroll
+                    for (int h = 0; h < RG; ++h) cfma((h & 1) ? p1 : p0, cconj(a[g + h]), xi[h]);
+                }
+            sj = mk(quad_sum(p0.x + p1.x), quad_sum(p0.y + p1.y));
+            const int src = (lane & 28) + ((q2 + 1) & 3);
+            yj = mk(__shfl_sync(0xffffffffu, ay.x, src), __shfl_sync(0xffffffffu, ay.y, src));
+            const int own = (lane & 28) + q2;
+            xj = mk(__shfl_sync(0xffffffffu, xj.x, own), __shfl_sync(0xffffffffu, xj.y, own));
+            double t = (q == 0 && col) ? xj.x * sj.x + xj.y * sj.y : 0.0;
+            t += __shfl_xor_sync(0xffffffffu, t, 4);
+            t += __shfl_xor_sync(0xffffffffu, t, 8);
+            t += __shfl_xor_sync(0xffffffffu, t, 16);
+            if (lane == 0) s.red2[warp] = t;
+            if (j == k + 1 && q == 0) {
+                s.akk = yj.x;
+                s.s1 = sj;
             }
+        } else if (lane == 0) {
+            s.red2[warp] = 0.0;
         }
         __syncthreads();
         const double beta = s.beta[k];
-        const bool on = beta != 0.0 && j > k && j < n;
-        double2 pj = mk(0.0, 0.0), uj = mk(0.0, 0.0);
-        const int ii0 = (k + 1) >> 2;
-        if (warp * 8 + 7 > k) {  // the warp holds an active column
-            double2 p0 = mk(0.0, 0.0), p1 = mk(0.0, 0.0);
-            if (on) {
+        double2 uj = mk(0.0, 0.0), wj = mk(0.0, 0.0);
+        const double2 c = mk(-s.sub[k].x, -s.sub[k].y);  // phase(x_0) |x|
+        if (beta != 0.0 && warp * 8 + 7 > k) {
+            double uau = 0.0;
 #pragma unroll
-                for (int ii = 0; ii < NE; ++ii) {
-                    const int i = 4 * ii + q;
-                    if (ii >= ii0 && i > k && i < n) cfma((ii & 1) ? p1 : p0, cconj(a[ii]), u[i]);
-                }
-                uj = u[j];
+            for (int t = 0; t < NW; ++t) uau += s.red2[t];
+            const double2 s1 = s.s1;
+            uau += 2.0 * (c.x * s1.x + c.y * s1.y) + (c.x * c.x + c.y * c.y) * s.akk;
+            const double K = 0.5 * beta * beta * uau;
+            if (col) {
+                uj = j == k + 1 ? cadd(xj, c) : xj;
+                double2 pj = sj;
+                cfma(pj, c, cconj(yj));
+                wj = mk(beta * pj.x - K * uj.x, beta * pj.y - K * uj.y);
             }
-            pj = mk(quad_sum(p0.x + p1.x) * beta, quad_sum(p0.y + p1.y) * beta);
-            double kp = (q == 0) ? uj.x * pj.x + uj.y * pj.y : 0.0;
-            kp = warp_sum(kp);
-            if (lane == 0) s.red[b][warp] = kp;
-            if (on && q == 0) p[j] = pj;
-        } else if (lane == 0) {
-            s.red[b][warp] = 0.0;
+        }
+        if (col && q == 0) {
+            s.U[k * (n - 1) - k * (k - 1) / 2 + j - k - 1] = uj;
+            s.wb[j] = wj;
+            if (j == k + 1) x[j] = uj;
         }
         __syncthreads();
-        if (on) {
-            double kp = 0.0;
+        if (beta != 0.0 && col) {
+            // A -= u w^H + w u^H; rows up to k take part with garbage: nothing reads them again
+            const double2 cw = mk(-wj.x, wj.y), cu = mk(-uj.x, uj.y);
 #pragma unroll
-            for (int t = 0; t < NW; ++t) kp += s.red[b][t];
-            const double K = 0.5 * beta * kp;
-            const double2 cw = mk(pj.x - K * uj.x, -(pj.y - K * uj.y)), cu = cconj(uj);
+            for (int g = 0; g < NE; g += RG)
+                if (g + RG > kb) {
+                    double2 xi[RG], wi[RG];
 #pragma unroll
-            for (int ii = 0; ii < NE; ++ii) {
-                const int i = 4 * ii + q;
-                if (ii >= ii0 && i > k && i < n) {
-                    const double2 ui = u[i], pi = p[i];
-                    const double2 wi = mk(pi.x - K * ui.x, pi.y - K * ui.y);
-                    a[ii] = csub(a[ii], cmul(ui, cw));
-                    a[ii] = csub(a[ii], cmul(wi, cu));
+                    for (int h = 0; h < RG; ++h) {
+                        xi[h] = x[4 * (g + h) + q];
+                        wi[h] = s.wb[4 * (g + h) + q];
+                    }
+#pragma unroll
+                    for (int h = 0; h < RG; ++h) cfma(a[g + h], xi[h], cw);
+#pragma unroll
+                    for (int h = 0; h < RG; ++h) cfma(a[g + h], wi[h], cu);
                 }
-            }
         }
     }
+    __syncthreads();
     // the last two diagonal entries and the last subdiagonal
 #pragma unroll
     for (int ii = 0; ii < NE; ++ii) {
@@ -307,7 +372,7 @@ __global__ void __launch_bounds__(DcGeo<NE>::NT, DcGeo<NE>::BLOCKS)
     __syncthreads();
 
     // ---- real tridiagonal: e_i = |sub_i|, delta_{i+1} = delta_i sub_i / |sub_i| ----
-    double2* delta = s.ub[0];
+    double2* delta = s.xb[0];
     if (q == 0 && j < n) {
         double ej = 0.0;
         if (j + 1 < n) ej = modulus(s.sub[j]);
@@ -432,6 +497,7 @@ __global__ void __launch_bounds__(DcGeo<NE>::NT, DcGeo<NE>::BLOCKS)
             const bool live = !s.df[j];
             const int at = live ? lo + before : lo + k + (j - lo - before);
             s.nd[at] = j;
+            s.pc[at] = s.perm[j];
             if (live) {
                 s.dk[at] = s.ds[j];
                 s.zk[at] = s.zs[j];
@@ -486,15 +552,19 @@ __global__ void __launch_bounds__(DcGeo<NE>::NT, DcGeo<NE>::BLOCKS)
         for (int ii = 0; ii < NE; ++ii) acc[ii] = 0.0;
         if (root) {
             const bool mixed = s.nrot[lo] > 0;  // a rotation joined columns of both halves
+#pragma unroll 4
             for (int t = 0; t < k; ++t) {
-                const int c = s.perm[s.nd[lo + t]];
+                const int c = s.pc[lo + t];
                 const double v = s.S[t * LD + j];
                 const double* Qc = s.Q + q * LD + c;
                 // without rotations column c is zero outside its half
-                const int i0 = (c < mid || mixed ? lo : mid) >> 2, i1 = ((c >= mid || mixed ? hi : mid) + 3) >> 2;
+                const int i0 = c < mid || mixed ? lo : mid, i1 = c >= mid || mixed ? hi : mid;
 #pragma unroll
-                for (int ii = 0; ii < NE; ++ii)
-                    if (ii >= i0 && ii < i1) acc[ii] = fma(Qc[4 * ii * LD], v, acc[ii]);
+                for (int g = 0; g < NE; g += 2)  // rows 4 g .. 4 g + 7 of the four lanes
+                    if (4 * g + 8 > i0 && 4 * g < i1) {
+                        acc[g] = fma(Qc[4 * g * LD], v, acc[g]);
+                        acc[g + 1] = fma(Qc[4 * (g + 1) * LD], v, acc[g + 1]);
+                    }
             }
         } else if (on) {
             const int at = s.nd[j], c = s.perm[at];
@@ -553,20 +623,34 @@ __global__ void __launch_bounds__(DcGeo<NE>::NT, DcGeo<NE>::BLOCKS)
     for (int k = n - 3; k >= 0; --k) {
         const double beta = s.beta[k];
         if (beta == 0.0) continue;
-        const double2* Uk = s.U + (size_t)k * (n - 1) - (size_t)k * (k - 1) / 2 - (k + 1);
-        const int ii0 = (k + 1) >> 2;
+        const double2* Uk = s.U + (k * (n - 1) - k * (k - 1) / 2 - (k + 1));
+        const int kb = k >> 2;
         double2 t0 = mk(0.0, 0.0), t1 = mk(0.0, 0.0);
 #pragma unroll
-        for (int ii = 0; ii < NE; ++ii) {
-            const int i = 4 * ii + q;
-            if (ii >= ii0 && i > k && i < n) cfma((ii & 1) ? t1 : t0, cconj(Uk[i]), a[ii]);
-        }
-        const double2 t = mk(beta * quad_sum(t0.x + t1.x), beta * quad_sum(t0.y + t1.y));
+        for (int g = 0; g < NE; g += RG)
+            if (g + RG > kb) {
+                double2 u[RG];
 #pragma unroll
-        for (int ii = 0; ii < NE; ++ii) {
-            const int i = 4 * ii + q;
-            if (ii >= ii0 && i > k && i < n) a[ii] = csub(a[ii], cmul(Uk[i], t));
-        }
+                for (int h = 0; h < RG; ++h) {
+                    const int i = 4 * (g + h) + q;
+                    u[h] = (i > k && i < n) ? Uk[i] : mk(0.0, 0.0);
+                }
+#pragma unroll
+                for (int h = 0; h < RG; ++h) cfma((h & 1) ? t1 : t0, cconj(u[h]), a[g + h]);
+            }
+        const double2 t = mk(-beta * quad_sum(t0.x + t1.x), -beta * quad_sum(t0.y + t1.y));
+#pragma unroll
+        for (int g = 0; g < NE; g += RG)
+            if (g + RG > kb) {
+                double2 u[RG];
+#pragma unroll
+                for (int h = 0; h < RG; ++h) {
+                    const int i = 4 * (g + h) + q;
+                    u[h] = (i > k && i < n) ? Uk[i] : mk(0.0, 0.0);
+                }
+#pragma unroll
+                for (int h = 0; h < RG; ++h) cfma(a[g + h], u[h], t);
+            }
     }
     if (j < n) {
         if (q == 0) wk[rank] = ldexp(dj, ex);
