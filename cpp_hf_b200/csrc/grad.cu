@@ -14,10 +14,11 @@
 #include "dm.cuh"
 #include "eigh.cuh"
 #include "mu.cuh"
+#include "mma64.cuh"
 #include "team.cuh"
 
 #include <algorithm>
-#include <mutex>
+#include <type_traits>
 #include <string>
 
 namespace cpphf {
@@ -205,12 +206,9 @@ __global__ void k_entropy_bwd(const double* __restrict__ p, const double* __rest
 // -w_k f'_i A / Z on the diagonal with A = sum_{k,i} Re(G~_ii) f'_i and
 // Z = sum_k w_k sum_i f'_i.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double fd_divided(double ei, double ej, double mu, double T) {
+__device__ __forceinline__ double fd_divided(double ei, double ej, double fi, double fj, double mu, double T) {
     const double s = (ei - ej) / (2.0 * T);
-    if (fabs(s) > 1.0e-3) {
-        const double fi = expit_g((mu - ei) / T), fj = expit_g((mu - ej) / T);
-        return (fi - fj) / (ei - ej);
-    }
+    if (fabs(s) > 1.0e-3) return (fi - fj) / (ei - ej);
     // f(x) = (1 - tanh(a))/2 with a = (e - mu)/(2T):
     // f_i - f_j = -sinh(a_i - a_j) / (2 cosh a_i cosh a_j), cosh a_i cosh a_j = (cosh(a_i + a_j) + cosh s)/2
     const double ssum = (ei + ej - 2.0 * mu) / (2.0 * T);
@@ -219,41 +217,21 @@ __device__ __forceinline__ double fd_divided(double ei, double ej, double mu, do
     return -sinhc / (2.0 * T * (cosh(ssum) + cosh(s)));
 }
 
-template <bool WARP>
-__global__ void k_dff_bwd_rotate(const double2* __restrict__ V, const double* __restrict__ eps,
-                                 const double* __restrict__ mu, double T, const double* __restrict__ w,
-                                 const double2* __restrict__ G, double2* __restrict__ Gt, int64_t nk, int nb,
-                                 ReduceWs* R, double* AZ) {
-    extern __shared__ __align__(16) unsigned char raw[];
+// A = sum_k,i f'(eps_ki) Re M_ii and Z = sum_k,i w_k f'(eps_ki) of M = V^H G V (the
+// diagonal of its Hermitian part)
+__global__ void k_dff_sums(const double2* __restrict__ M, const double* __restrict__ eps, const double* __restrict__ mu,
+                           double T, const double* __restrict__ w, int64_t nk, int nb, ReduceWs* R, double* AZ) {
     __shared__ double red[64];
-    Team<WARP> t;
-    const int ld = nb + 1;
-    double2* Vs = team_mats<WARP>(raw, nb, 3, 0, t.team);
-    double2* Gs = Vs + team_mat_elems(nb);
-    double2* Ts = Gs + team_mat_elems(nb);
     const double m = *mu;
     double v[2] = {0.0, 0.0};
-    for (int64_t k = (int64_t)blockIdx.x * t.nteams + t.team; k < nk; k += (int64_t)gridDim.x * t.nteams) {
-        tload<WARP>(Vs, V + (size_t)k * nb * nb, nb, t);
-        const double2* Gk = G + (size_t)k * nb * nb;
-        for (int e = t.tid; e < nb * nb; e += t.nt) {  // herm(G)
-            const int i = e / nb, j = e - i * nb;
-            const double2 a = Gk[e], b = Gk[(size_t)j * nb + i];
-            Gs[i * ld + j] = mk(0.5 * (a.x + b.x), 0.5 * (a.y - b.y));
-        }
-        t.sync();
-        tmm<false, false, WARP>(Ts, Gs, Vs, nb, t);  // herm(G) V
-        t.sync();
-        tmm<true, false, WARP>(Gs, Vs, Ts, nb, t);   // V^H herm(G) V
-        t.sync();
-        tstore<WARP>(Gt + (size_t)k * nb * nb, Gs, nb, t);
-        for (int i = t.tid; i < nb; i += t.nt) {
-            const double f = expit_g((m - eps[(size_t)k * nb + i]) / T);
-            const double fp = -f * (1.0 - f) / T;
-            v[0] += Gs[i * ld + i].x * fp;
-            v[1] += w[k] * fp;
-        }
-        t.sync();
+    const int64_t n = nk * nb;
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t k = e / nb;
+        const int i = (int)(e - k * nb);
+        const double f = expit_g((m - eps[e]) / T);
+        const double fp = -f * (1.0 - f) / T;
+        v[0] += M[(size_t)e * nb + i].x * fp;
+        v[1] += w[k] * fp;
     }
     double out[2];
     if (reduce_last_block<2>(v, R->part, &R->counter, out, red) && threadIdx.x == 0) {
@@ -262,53 +240,110 @@ __global__ void k_dff_bwd_rotate(const double2* __restrict__ V, const double* __
     }
 }
 
-template <bool WARP>
-__global__ void k_dff_bwd_apply(const double2* __restrict__ V, const double* __restrict__ eps,
-                                const double* __restrict__ mu, double T, const double* __restrict__ w,
-                                const double* __restrict__ AZ, double2* gF, int64_t nk, int nb) {
+// gF = V X V^H in place of M, X_ij = herm(M)_ij (f_i - f_j) / (eps_i - eps_j), less the
+// chemical-potential term on the diagonal, on the FP64 tensor cores (mma64.cuh): the
+// rows of X are formed eight at a time into a double-buffered chunk, the B operand of
+// T = V X, and T, in registers, is the A operand of T V^H, whose column tiles are
+// formed in two halves.  Bound by the divided differences and the FP64 products; the
+// team kernels it replaces (with the rotation that gives M) read both operands of
+// every FMA from shared memory: 2304 k-points of nb = 32, 157 + 186 us -> 49 + 9 + 112.
+template <int NT>
+constexpr size_t dff_smem() {
+    return sizeof(double2) * (MmaGeo<NT>::MAT + 2 * 8 * (size_t)MmaGeo<NT>::LD) + sizeof(double) * 2 * MmaGeo<NT>::NP;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(MmaGeo<NT>::THREADS, MmaGeo<NT>::BLOCKS)
+    k_dff_apply(const double2* __restrict__ V, const double* __restrict__ eps, const double* __restrict__ mu, double T,
+                const double* __restrict__ w, const double* __restrict__ AZ, double2* gF, int64_t nk, int nb) {
+    constexpr int LD = MmaGeo<NT>::LD, GR = MmaGeo<NT>::GROUPS, GT = MmaGeo<NT>::GT;
     extern __shared__ __align__(16) unsigned char raw[];
-    Team<WARP> t;
-    const int ld = nb + 1;
-    double2* Vs = team_mats<WARP>(raw, nb, 3, nb, t.team);
-    double2* Ms = Vs + team_mat_elems(nb);
-    double2* Ts = Ms + team_mat_elems(nb);
-    double* es = reinterpret_cast<double*>(Ts + team_mat_elems(nb));
-    const double m = *mu;
-    const double Z = AZ[1];
+    const int grp = threadIdx.x / GT, gt = threadIdx.x % GT, wp = gt >> 5, lane = gt & 31, r = lane >> 2, t = lane & 3;
+    double2* Vs = reinterpret_cast<double2*>(raw + dff_smem<NT>() * grp);
+    double2* Xs = Vs + MmaGeo<NT>::MAT;
+    double *es = reinterpret_cast<double*>(Xs + 2 * 8 * LD), *fs = es + MmaGeo<NT>::NP;
+    const double m = *mu, Z = AZ[1];
     const double ratio = (fabs(Z) > 1.0e-300) ? AZ[0] / Z : 0.0;
-    for (int64_t k = (int64_t)blockIdx.x * t.nteams + t.team; k < nk; k += (int64_t)gridDim.x * t.nteams) {
-        tload<WARP>(Vs, V + (size_t)k * nb * nb, nb, t);
-        tload<WARP>(Ms, gF + (size_t)k * nb * nb, nb, t);
-        for (int i = t.tid; i < nb; i += t.nt) es[i] = eps[(size_t)k * nb + i];
-        t.sync();
-        for (int e = t.tid; e < nb * nb; e += t.nt) {
-            const int i = e / nb, j = e - i * nb;
-            double d = fd_divided(es[i], es[j], m, T);
-            double2 x = cscale(Ms[i * ld + j], d);
-            if (i == j) {
-                const double f = expit_g((m - es[i]) / T);
-                x.x -= w[k] * (-f * (1.0 - f) / T) * ratio;
-            }
-            Ms[i * ld + j] = x;
+    for (int i = gt; i < 2 * 8 * LD; i += GT) Xs[i] = mk(0.0, 0.0);  // the padding
+    for (int64_t k = (int64_t)blockIdx.x * GR + grp; k < nk; k += (int64_t)gridDim.x * GR) {
+        const size_t off = (size_t)k * nb * nb;
+        mma_load_smem<NT>(Vs, V + off, nb, gt);
+        for (int i = gt; i < nb; i += GT) {
+            es[i] = eps[(size_t)k * nb + i];
+            fs[i] = expit_g((m - es[i]) / T);
         }
-        t.sync();
-        tmm<false, true, WARP>(Ts, Ms, Vs, nb, t);   // M V^H
-        t.sync();
-        tmm<false, false, WARP>(Ms, Vs, Ts, nb, t);  // V M V^H
-        t.sync();
-        tstore<WARP>(gF + (size_t)k * nb * nb, Ms, nb, t);
-        t.sync();
+        group_sync<NT>();
+        const double wk = w[k];
+        double2 c[NT][2];
+        mma_zero<NT>(c);
+#pragma unroll 1
+        for (int kt = 0; kt < NT; ++kt) {
+            double2* X = Xs + (kt & 1) * 8 * LD;
+            for (int e = gt; e < 8 * nb; e += GT) {
+                const int il = e / nb, j = e - il * nb, i = 8 * kt + il;
+                double2 x = mk(0.0, 0.0);
+                if (i < nb) {
+                    const double2 a = gF[off + (size_t)i * nb + j], b = gF[off + (size_t)j * nb + i];
+                    x = cscale(mk(0.5 * (a.x + b.x), 0.5 * (a.y - b.y)), fd_divided(es[i], es[j], fs[i], fs[j], m, T));
+                    if (i == j) {
+                        const double f = fs[i];
+                        x.x -= wk * (-f * (1.0 - f) / T) * ratio;
+                    }
+                }
+                X[il * LD + j] = x;
+            }
+            group_sync<NT>();  // chunk kt is there; chunk kt - 1 is read by all before it is overwritten
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const double2 av = Vs[(8 * wp + r) * LD + 8 * kt + 2 * t + s];
+#pragma unroll
+                for (int j = 0; j < NT; ++j) zmma(c[j], av, X[(2 * t + s) * LD + 8 * j + r]);
+            }
+        }
+        const int row = 8 * wp + r;
+        auto half = [&](auto j0c, auto ncc) {
+            constexpr int J0 = decltype(j0c)::value, NC = decltype(ncc)::value;
+            double2 o[NC][2];
+            mma_zero<NC>(o);
+#pragma unroll
+            for (int kt = 0; kt < NT; ++kt)
+#pragma unroll
+                for (int s = 0; s < 2; ++s)
+#pragma unroll
+                    for (int j = 0; j < NC; ++j)
+                        zmma(o[j], c[kt][s], cconj(Vs[(8 * (J0 + j) + r) * LD + 8 * kt + 2 * t + s]));
+            if (row < nb) {
+#pragma unroll
+                for (int j = 0; j < NC; ++j)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int col = 8 * (J0 + j) + 2 * t + h;
+                        if (col < nb) gF[off + (size_t)row * nb + col] = o[j][h];
+                    }
+            }
+        };
+        half(std::integral_constant<int, 0>{}, std::integral_constant<int, (NT + 1) / 2>{});
+        if constexpr (NT > 1)
+            half(std::integral_constant<int, (NT + 1) / 2>{}, std::integral_constant<int, NT / 2>{});
+        group_sync<NT>();
     }
 }
 
-void init_grad_attrs() {
-    static std::once_flag once;
-    std::call_once(once, [] {
-        raise_smem(k_dff_bwd_rotate<true>);
-        raise_smem(k_dff_bwd_rotate<false>);
-        raise_smem(k_dff_bwd_apply<true>);
-        raise_smem(k_dff_bwd_apply<false>);
-    });
+template <int NT>
+int launch_dff_apply(const double2* V, const double* eps, const double* mu, double T, const double* w, const double* AZ,
+                     double2* gF, int64_t nk, int nb, cudaStream_t st) {
+    constexpr int GR = MmaGeo<NT>::GROUPS;
+    static const int ctas = [] {
+        raise_smem(k_dff_apply<NT>);
+        int per = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_dff_apply<NT>, MmaGeo<NT>::THREADS, GR * dff_smem<NT>());
+        (void)cudaGetLastError();
+        return std::max(per, 1) * num_sms();
+    }();
+    k_dff_apply<NT><<<(unsigned)std::min<int64_t>((nk + GR - 1) / GR, ctas), MmaGeo<NT>::THREADS, GR * dff_smem<NT>(), st>>>(
+        V, eps, mu, T, w, AZ, gF, nk, nb);
+    CPPHF_LAUNCH_CHECK("density_from_fock backward");
+    return CPPHF_OK;
 }
 
 int check_sizes(int64_t nk, int64_t nb) {
@@ -389,19 +424,26 @@ int density_from_fock_backward(const double2* V, const double* eps, const double
     if (!(T > 0.0)) return fail(CPPHF_ERR_INVALID, "density_from_fock_backward: T must be positive");
     if (!ws || wsb < density_from_fock_backward_workspace_bytes())
         return fail(CPPHF_ERR_INVALID, "density_from_fock_backward: workspace too small");
-    init_grad_attrs();
     ReduceWs* R = static_cast<ReduceWs*>(ws);
     double* AZ = reinterpret_cast<double*>(static_cast<unsigned char*>(ws) + sizeof(ReduceWs));
     CPPHF_CUDA(cudaMemsetAsync(&R->counter, 0, sizeof(unsigned), st));
-    TeamLaunch L = team_launch(nk, (int)nb);
-    L.grid = std::min<unsigned>(L.grid, kGradMaxBlocks);
     const int n = (int)nb;
-    {
-        const int nb = n;  // for TEAM_DISPATCH's shared-memory size
-        TEAM_DISPATCH(L, k_dff_bwd_rotate, 3, 0, V, eps, mu, T, w, G, gF, nk, n, R, AZ);
-        TEAM_DISPATCH(L, k_dff_bwd_apply, 3, nb, V, eps, mu, T, w, AZ, gF, nk, n);
+    CPPHF_TRY(dm_rotate(V, G, gF, nullptr, nk, n, st));
+    k_dff_sums<<<red_grid(nk * nb), 256, 0, st>>>(gF, eps, mu, T, w, nk, n, R, AZ);
+    CPPHF_LAUNCH_CHECK("density_from_fock backward sums");
+    switch ((n + 7) / 8) {
+        case 1: return launch_dff_apply<1>(V, eps, mu, T, w, AZ, gF, nk, n, st);
+        case 2: return launch_dff_apply<2>(V, eps, mu, T, w, AZ, gF, nk, n, st);
+        case 3: return launch_dff_apply<3>(V, eps, mu, T, w, AZ, gF, nk, n, st);
+        case 4: return launch_dff_apply<4>(V, eps, mu, T, w, AZ, gF, nk, n, st);
+        case 5: return launch_dff_apply<5>(V, eps, mu, T, w, AZ, gF, nk, n, st);
+        case 6: return launch_dff_apply<6>(V, eps, mu, T, w, AZ, gF, nk, n, st);
+        case 7: return launch_dff_apply<7>(V, eps, mu, T, w, AZ, gF, nk, n, st);
+        case 8: return launch_dff_apply<8>(V, eps, mu, T, w, AZ, gF, nk, n, st);
+        case 9: return launch_dff_apply<9>(V, eps, mu, T, w, AZ, gF, nk, n, st);
+        default: break;
     }
-    return CPPHF_OK;
+    return fail(CPPHF_ERR_UNSUPPORTED, "nb too large for the per-k kernels");
 }
 
 }  // namespace cpphf
