@@ -47,17 +47,6 @@ constexpr int kColsVR = 0;
 constexpr int kColsConjVR = 1;
 constexpr int kColsForwardOnly = 2;
 
-// channel -> (row, col) of the HCP packing (upper triangle, row-major).
-__device__ __forceinline__ void hcp_pair(int ch, int nb, int& i, int& j) {
-    int r = 0, c = ch;
-    while (c >= nb - r) {
-        c -= nb - r;
-        ++r;
-    }
-    i = r;
-    j = r + c;
-}
-
 __device__ __forceinline__ void build_map(int* map, int chunk0, int CB, int C, int nb, int hcp) {
     for (int c = threadIdx.x; c < CB; c += blockDim.x) {
         const int ch = chunk0 + c;
@@ -65,9 +54,10 @@ __device__ __forceinline__ void build_map(int* map, int chunk0, int CB, int C, i
         if (ch < C) {
             if (hcp) {
                 int i, j;
-                hcp_pair(ch, nb, i, j);
-                off = i * nb + j;
-                mir = (i != j) ? j * nb + i : -1;
+                if (hcp_pair(ch, nb, hcp, i, j)) {
+                    off = i * nb + j;
+                    mir = (i != j) ? j * nb + i : -1;
+                }
             } else {
                 off = ch;
             }
@@ -777,7 +767,10 @@ struct Spec {
                 }
             }
         }
-        const Launch L = plan_launch(N1 > N2 ? N1 : N2, g.C, sizeof(Cx), N1 * N2, false);
+        // a tile of the 4 x 4 packing per CTA (half of one where the line needs the lanes)
+        constexpr int lanes = N1 > N2 ? N1 : N2;
+        const Launch L = plan_launch(lanes, g.C, sizeof(Cx), N1 * N2, false,
+                                     g.hcp == 2 ? (lanes <= 16 ? 16 : 8) * lanes : kTargetThreads);
         k_rows_fwd_s<Cx, N1, N2><<<dim3(g.n0, L.nchunk), L.threads, L.smem, st>>>(P, refP, T, g, L.CB);
         CPPHF_LAUNCH_CHECK("exchange rows forward");
         return CPPHF_OK;
@@ -966,6 +959,20 @@ size_t exchange_t_bytes(int64_t nk1, int64_t nk2, int64_t nb, int hcp, int preci
 // T when it does not alias Sigma (0 for the full FP64 form).
 size_t exchange_workspace_bytes(int64_t nk1, int64_t nk2, int64_t nb, int hcp, int precision) {
     return exchange_t_bytes(nk1, nk2, nb, hcp, precision);
+}
+
+int exchange_hcp_two_passes(const double2* P, const double2* refP, const double2* VR, double2* T, const ExchangeGeom& g,
+                            cudaStream_t st) {
+    CPPHF_TRY(pass_rows_fwd<double2>(P, refP, T, g, st));
+    ExchangeGeom gc = g;  // the columns pass does not see the packing
+    gc.hcp = 0;
+    return pass_cols<double2>(T, VR, gc, kColsVR, st);
+}
+
+bool hcp_tiled(int64_t n0, int64_t n1, int64_t nb) {
+    if (nb <= 8 || nb > 4096 || n0 > 65535 || n1 > 65535 || split_of((int)n1).n1 == 0) return false;
+    const int64_t tiled = hcp_channels(2, (int)nb), tri = hcp_channels(1, (int)nb), field = n0 * n1 * nb * nb;
+    return field >= (int64_t)1 << 22 && (10 * tiled <= 13 * tri || (10 * tiled <= 16 * tri && field >= (int64_t)1 << 23));
 }
 
 int exchange_columns(void* T, const double2* VR, const ExchangeGeom& g, int precision, cudaStream_t st) {

@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "exchange.cuh"
 #include "fock.cuh"
+#include "fock_mesh.cuh"
 #include "superlattice.cuh"
 #include "team.cuh"
 
@@ -339,7 +340,8 @@ FockWs fock_ws_layout(const cpphf_kernel* K) {
     L.off_sc = take(sizeof(double2) * nb2);
     L.off_hd = take(sizeof(double) * nb);
     const int hcp = (K->exchange_hcp && K->dv == 1) ? 1 : 0;
-    L.off_exch = take(exchange_workspace_bytes(K->nk1, K->nk2, K->nb, hcp, K->exchange_precision));
+    L.off_exch = take(std::max(exchange_workspace_bytes(K->nk1, K->nk2, K->nb, hcp, K->exchange_precision),
+                               fock_mesh_bytes(K)));
     L.off_pack = take(packed_fock_workspace_bytes(K));
     L.sl_bytes = 0;
     L.off_sl = L.off_slh = L.off_rho = o;
@@ -425,6 +427,22 @@ int build_fock(const cpphf_kernel* K, const double2* P, double2* Sigma, double2*
         return build_fock_packed(K, P, Sigma, F, (K->include_hartree && !slh) ? hd : nullptr,
                                  (K->has_contact || slh) ? SC : nullptr, need_pre ? rho_bar : nullptr, energy,
                                  Hdense, part, counter, W + L.off_pack, wsb - L.off_pack, st);
+    }
+    if (fock_mesh_eligible(K)) {
+        MeshOut o;
+        o.h = static_cast<const double2*>(K->h);
+        o.P = P;
+        o.refP = refP;
+        o.w = K->w2d;
+        o.hd = K->include_hartree ? hd : nullptr;
+        o.SC = K->has_contact ? SC : nullptr;
+        o.Sigma = Sigma;
+        o.F = F;
+        o.Hdense = Hdense;
+        o.energy = energy;
+        o.part = part;
+        o.counter = reinterpret_cast<unsigned*>(W + L.off_counter);
+        return build_fock_mesh(K, o, W + L.off_exch, st);
     }
     if (!Sigma) return fail(CPPHF_ERR_INVALID, "build_fock: null Sigma");
     if (sl_fock(K)) {

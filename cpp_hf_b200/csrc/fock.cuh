@@ -2,6 +2,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "fock_mesh.cuh"
 
 namespace cpphf {
 
@@ -34,7 +35,9 @@ size_t solver_pack_bytes(const cpphf_kernel* K);
 int solver_pack(const cpphf_kernel* K, cpphf_kernel* out, void* ws, cudaStream_t st);
 // build_fock workspace bytes for K once its packed fields exist.
 size_t fock_bytes_packed_kernel(const cpphf_kernel* K);
-// The Sigma a solver passes to build_fock: none when the packed build runs.
-inline double2* solver_sigma(const cpphf_kernel* K, double2* Sig) { return packed_fock_eligible(K) ? nullptr : Sig; }
+// The Sigma a solver passes to build_fock: none when a build that fuses the assembly runs.
+inline double2* solver_sigma(const cpphf_kernel* K, double2* Sig) {
+    return packed_fock_eligible(K) || fock_mesh_eligible(K) ? nullptr : Sig;
+}
 
 }  // namespace cpphf

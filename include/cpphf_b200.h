@@ -216,7 +216,8 @@ int cpphf_kernel_pack(const cpphf_kernel* K, void* VR_packed, void* h_packed, vo
  * k-independent Hartree diagonal hartree_diag (nb) and the energy
  * E = sum_k w_k Re Tr[h P + (Sigma + H)(P - refP)/2] (device scalar *energy).
  * H_dense (complex128 field, may be NULL) receives the dense Hartree term.
- * Sigma may be NULL when K's Hermitian packing applies (see cpphf_kernel).
+ * Sigma may be NULL when K's Hermitian packing applies (see cpphf_kernel) or the
+ * build of many bands with a scalar V fuses the assembly; solvers then skip it.
  * ---------------------------------------------------------------------- */
 size_t cpphf_build_fock_workspace_bytes(const cpphf_kernel* K);
 int cpphf_build_fock(const cpphf_kernel* K, const void* P, void* Sigma, void* F,
