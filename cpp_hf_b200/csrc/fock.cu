@@ -1,7 +1,7 @@
 // Fock assembly and Hartree-Fock energy (cpp_hf fock.hpp:34-383).
 //
 //   pre      (only with Hartree or contact terms): rho_bar = sum_k w_k (P - refP)
-//            by per-block partials + fixed-order final sum; then
+//            by per-block partials + fixed-order sums in the last blocks; then
 //            hartree_diag = HH n_vec (n_vec = Re diag rho_bar) and the contact
 //            self-energy SC = sum_t g_t [Oi tr(Oj rho_bar) - Oi rho_bar Oj].
 //   exchange Sigma = -IFFT2[FFT2(P - refP) VR] (exchange.cu), or zero.
@@ -30,92 +30,131 @@ namespace cpphf {
 namespace {
 
 constexpr int kAsmThreads = 256;
-constexpr int kRedThreads = 256;
 constexpr int kMaxPartials = kFockMaxPartials;
 constexpr int kAsmMaxStages = 4;
 constexpr int kTileElems = 1024;  // k-blocks of at most this many elements take the bulk-pipelined assembly
 
-// rho_bar partials: grid (Gk, ceil(nb2 / CH)), CH channels per block, lanes =
-// blockDim / CH k-lanes.
-__global__ void k_rho_bar_partial(const double2* __restrict__ P, const double2* __restrict__ refP,
-                                  const double* __restrict__ w, int64_t nk, int nb2, int CH,
-                                  double2* __restrict__ part) {
-    __shared__ double2 acc_sh[kRedThreads];
-    const int lanes = blockDim.x / CH;
-    const int c_local = threadIdx.x % CH, lane = threadIdx.x / CH;
-    const int c = blockIdx.y * CH + c_local;
-    const int Gk = gridDim.x;
-    const int64_t per = (nk + Gk - 1) / Gk;
-    const int64_t k0 = (int64_t)blockIdx.x * per, k1 = min(nk, k0 + per);
+// rho_bar, the Hartree diagonal and the contact self-energy SC in one launch.  Grid
+// (Gk, slices of CH channels), 1024 threads: CH channels by 1024 / CH k-lanes, each
+// lane's points eight loads at a time.  The last block of a slice sums its Gk partials,
+// the last block of all forms hd = HH Re diag rho_bar and
+// SC = sum_t g [Oi tr(Oj rho_bar) - (Oi rho_bar) Oj] (all sums in a fixed order).
+// Bound by HBM for large meshes (P and refP read once), by the chain of the two
+// tickets for small ones.  Whole builds with refP and two contact terms, us, against
+// 256-thread partials summed serially by a second, single-block kernel: 192 x 192,
+// nb = 8: 127/159; 75 x 98, nb = 5: 61/74; 48 x 48, nb = 2: 42/45; 36 x 36, nb = 64:
+// 399/6575 (the products there were formed entry by entry, nb^4).
+constexpr int kRhoThreads = 1024;
+constexpr int kRhoChannels = 256;
+
+__global__ void __launch_bounds__(kRhoThreads)
+    k_hartree_contact(const double2* __restrict__ P, const double2* __restrict__ refP, const double* __restrict__ w,
+                      int64_t nk, int nb, int CH, double2* part, unsigned* counter, const double* __restrict__ HH,
+                      int include_hartree, int has_contact, int n_contact, const double* __restrict__ cg,
+                      const double2* __restrict__ Oi, const double2* __restrict__ Oj, double2* rho_bar,
+                      double* __restrict__ hd, double2* SC) {
+    __shared__ double2 acc_sh[kRhoThreads];
+    __shared__ double red[2 * kRhoThreads / 32];
+    __shared__ int last;
+    const int nb2 = nb * nb, Gk = gridDim.x, tid = threadIdx.x;
+    const int lanes = kRhoThreads / CH, cl = tid % CH, lane = tid / CH;
+    const int c = blockIdx.y * CH + cl;
+    const bool live = lane < lanes && c < nb2;
+    const int64_t per = (nk + Gk - 1) / Gk, k0 = blockIdx.x * per, k1 = min(nk, k0 + per);
     double2 acc = mk(0.0, 0.0);
-    if (lane < lanes && c < nb2) {
-        for (int64_t k = k0 + lane; k < k1; k += lanes) {
-            double2 v = P[(size_t)k * nb2 + c];
-            if (refP) v = csub(v, refP[(size_t)k * nb2 + c]);
-            const double wk = w[k];
-            acc.x += wk * v.x;
-            acc.y += wk * v.y;
+    if (live) {
+        int64_t k = k0 + lane;
+        for (; k + 3 * lanes < k1; k += 4 * lanes) {
+            double2 v[4], r[4];
+            double wk[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const size_t at = (size_t)(k + u * lanes) * nb2 + c;
+                v[u] = P[at];
+                r[u] = refP ? ld_stream(refP + at) : mk(0.0, 0.0);
+                wk[u] = w[k + u * lanes];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                acc.x += wk[u] * (v[u].x - r[u].x);
+                acc.y += wk[u] * (v[u].y - r[u].y);
+            }
+        }
+        for (; k < k1; k += lanes) {
+            const size_t at = (size_t)k * nb2 + c;
+            double2 v = P[at];
+            if (refP) v = csub(v, ld_stream(refP + at));
+            acc.x += w[k] * v.x;
+            acc.y += w[k] * v.y;
         }
     }
-    acc_sh[threadIdx.x] = acc;
+    acc_sh[tid] = acc;
     __syncthreads();
-    if (lane == 0 && c < nb2) {
-        double2 s = acc;
-        for (int l = 1; l < lanes; ++l) s = cadd(s, acc_sh[l * CH + c_local]);
-        part[(size_t)blockIdx.x * nb2 + c] = s;
-    }
-}
-
-// Final: rho_bar, hartree_diag and the contact self-energy SC (single block).
-__global__ void k_hartree_contact(const double2* __restrict__ part, int Gk, int nb,
-                                  const double* __restrict__ HH, int include_hartree,
-                                  int has_contact, int n_contact, const double* __restrict__ cg,
-                                  const double2* __restrict__ Oi, const double2* __restrict__ Oj,
-                                  double2* __restrict__ rho_bar, double* __restrict__ hd,
-                                  double2* __restrict__ SC) {
-    const int nb2 = nb * nb;
-    for (int c = threadIdx.x; c < nb2; c += blockDim.x) {
-        double2 s = mk(0.0, 0.0);
-        for (int b = 0; b < Gk; ++b) s = cadd(s, part[(size_t)b * nb2 + c]);
-        rho_bar[c] = s;
+    if (lane == 0 && live) {
+        for (int l = 1; l < lanes; ++l) acc = cadd(acc, acc_sh[l * CH + cl]);
+        st_l2(part + (size_t)blockIdx.x * nb2 + c, acc);
+        __threadfence();
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) {
+    if (tid == 0) last = atomicAdd(counter + 1 + blockIdx.y, 1u) == (unsigned)Gk - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    acc = mk(0.0, 0.0);
+    if (live) {
+#pragma unroll 4
+        for (int b = lane; b < Gk; b += lanes) acc = cadd(acc, ld_l2(part + (size_t)b * nb2 + c));
+    }
+    acc_sh[tid] = acc;
+    __syncthreads();
+    if (lane == 0 && live) {
+        for (int l = 1; l < lanes; ++l) acc = cadd(acc, acc_sh[l * CH + cl]);
+        st_l2(rho_bar + c, acc);
+        __threadfence();
+    }
+    __syncthreads();
+    if (tid == 0) last = atomicAdd(counter, 1u) == gridDim.y - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int i = tid / 32; i < nb; i += kRhoThreads / 32) {
         double s = 0.0;
         if (include_hartree)
-            for (int j = 0; j < nb; ++j) s += HH[i * nb + j] * rho_bar[j * nb + j].x;
-        hd[i] = s;
+            for (int j = tid & 31; j < nb; j += 32) s += HH[i * nb + j] * ld_l2(rho_bar + j * nb + j).x;
+        s = warp_sum(s);
+        if ((tid & 31) == 0) hd[i] = s;
     }
     if (!has_contact) return;
-    // SC_ij = sum_t g [Oi_ij tr(Oj rho) - (Oi rho Oj)_ij]
-    __shared__ double2 tr_sh[64];
-    for (int c = threadIdx.x; c < nb2; c += blockDim.x) SC[c] = mk(0.0, 0.0);
-    __syncthreads();
+    double2* orho = part;  // the partials are summed: their space takes Oi rho_bar
+    for (int e = tid; e < nb2; e += kRhoThreads) SC[e] = mk(0.0, 0.0);
     for (int t = 0; t < n_contact; ++t) {
         const double g = cg[t];
         if (g == 0.0) continue;
         const double2* oi = Oi + (size_t)t * nb2;
         const double2* oj = Oj + (size_t)t * nb2;
-        if (threadIdx.x == 0) {
-            double2 tr = mk(0.0, 0.0);
-            for (int i = 0; i < nb; ++i)
-                for (int j = 0; j < nb; ++j) tr = cadd(tr, cmul(oj[i * nb + j], rho_bar[j * nb + i]));
-            tr_sh[0] = tr;
+        double tr[2] = {0.0, 0.0};
+        for (int e = tid; e < nb2; e += kRhoThreads) {
+            const int i = e / nb, j = e - i * nb;
+            const double2 x = cmul(oj[e], ld_l2(rho_bar + j * nb + i));
+            tr[0] += x.x;
+            tr[1] += x.y;
+            double2 o = mk(0.0, 0.0);
+#pragma unroll 8
+            for (int m = 0; m < nb; ++m) o = cadd(o, cmul(oi[i * nb + m], ld_l2(rho_bar + m * nb + j)));
+            orho[e] = o;
         }
+        block_sum<2>(tr, red);
         __syncthreads();
-        const double2 tr = tr_sh[0];
-        for (int c = threadIdx.x; c < nb2; c += blockDim.x) {
-            const int i = c / nb, j = c - i * nb;
+        if (tid == 0) acc_sh[0] = mk(tr[0], tr[1]);
+        __syncthreads();
+        const double2 trace = acc_sh[0];
+        for (int e = tid; e < nb2; e += kRhoThreads) {
+            const int i = e / nb, j = e - i * nb;
             // herm = Oi * tr * g ; fk = -g * (Oi rho Oj)
-            const double2 herm = cscale(cmul(oi[c], tr), g);
-            double2 orho_oj = mk(0.0, 0.0);
-            for (int l = 0; l < nb; ++l) {
-                double2 orho = mk(0.0, 0.0);
-                for (int m = 0; m < nb; ++m) orho = cadd(orho, cmul(oi[i * nb + m], rho_bar[m * nb + l]));
-                orho_oj = cadd(orho_oj, cmul(orho, oj[l * nb + j]));
-            }
-            const double2 fk = cscale(orho_oj, -g);
-            SC[c] = cadd(SC[c], cadd(herm, fk));
+            double2 o = mk(0.0, 0.0);
+#pragma unroll 8
+            for (int l = 0; l < nb; ++l) o = cadd(o, cmul(orho[i * nb + l], oj[l * nb + j]));
+            SC[e] = cadd(SC[e], cadd(cscale(cmul(oi[e], trace), g), cscale(o, -g)));
         }
         __syncthreads();
     }
@@ -302,9 +341,9 @@ __global__ void k_sum_partials(const double* __restrict__ part, int n, double* _
 }
 
 struct FockWs {
-    size_t off_part, off_counter, off_rho_part, off_rho_bar, off_sc, off_hd, off_exch, off_pack, total;
+    size_t off_part, off_counter, off_rho_counter, off_rho_part, off_rho_bar, off_sc, off_hd, off_exch, off_pack, total;
     size_t off_sl, sl_bytes, off_slh, off_rho;
-    int Gasm, Gk;
+    int Gasm, Gk, CH, slices;
 };
 
 bool sl_fock(const cpphf_kernel* K) { return K->sl && K->sl->fock_active && K->include_exchange; }
@@ -326,7 +365,11 @@ FockWs fock_ws_layout(const cpphf_kernel* K) {
     const int64_t npair = nb * (nb + 1) / 2;
     const int64_t need = (nk * npair + kAsmThreads - 1) / kAsmThreads;
     L.Gasm = (int)std::max<int64_t>(1, std::min<int64_t>(need, std::min(kMaxPartials, 8 * num_sms())));
-    L.Gk = (int)std::max<int64_t>(1, std::min<int64_t>(nk, 2 * num_sms()));
+    // rho_bar: at least four points per lane, at most a block per SM (two per SM over several slices)
+    L.CH = (int)std::min<int64_t>(nb2, kRhoChannels);
+    L.slices = (int)((nb2 + L.CH - 1) / L.CH);
+    const int64_t lane_points = 4 * (kRhoThreads / L.CH), most = L.slices > 1 ? 2 * num_sms() / L.slices : num_sms();
+    L.Gk = (int)std::max<int64_t>(1, std::min<int64_t>((nk + lane_points - 1) / lane_points, most));
     size_t o = 0;
     auto take = [&](size_t bytes) {
         size_t at = o;
@@ -335,6 +378,7 @@ FockWs fock_ws_layout(const cpphf_kernel* K) {
     };
     L.off_part = take(sizeof(double) * kMaxPartials);
     L.off_counter = take(sizeof(unsigned));
+    L.off_rho_counter = take(sizeof(unsigned) * (1 + (size_t)L.slices));
     L.off_rho_part = take(sizeof(double2) * (size_t)L.Gk * nb2);
     L.off_rho_bar = take(sizeof(double2) * nb2);
     L.off_sc = take(sizeof(double2) * nb2);
@@ -407,16 +451,13 @@ int build_fock(const cpphf_kernel* K, const double2* P, double2* Sigma, double2*
     const bool need_pre = K->include_hartree || K->has_contact;
     const bool slh = sl_hart(K);
     if (need_pre) {
-        const int CH = std::min(nb2, kRedThreads);
-        dim3 grid(L.Gk, (nb2 + CH - 1) / CH);
-        k_rho_bar_partial<<<grid, kRedThreads, 0, st>>>(P, refP, K->w2d, nk, nb2, CH, rho_part);
-        CPPHF_LAUNCH_CHECK("rho_bar partial");
+        unsigned* rho_counter = reinterpret_cast<unsigned*>(W + L.off_rho_counter);
+        CPPHF_CUDA(cudaMemsetAsync(rho_counter, 0, sizeof(unsigned) * (1 + (size_t)L.slices), st));
         // the superlattice Hartree replaces the diagonal Hartree (fock.hpp:66-175)
-        k_hartree_contact<<<1, 256, 0, st>>>(rho_part, L.Gk, nb, K->HH, K->include_hartree && !slh,
-                                             K->has_contact, K->n_contact, K->contact_g,
-                                             static_cast<const double2*>(K->contact_Oi),
-                                             static_cast<const double2*>(K->contact_Oj), rho_bar,
-                                             hd, SC);
+        k_hartree_contact<<<dim3(L.Gk, L.slices), kRhoThreads, 0, st>>>(
+            P, refP, K->w2d, nk, nb, L.CH, rho_part, rho_counter, K->HH, K->include_hartree && !slh, K->has_contact,
+            K->n_contact, K->contact_g, static_cast<const double2*>(K->contact_Oi),
+            static_cast<const double2*>(K->contact_Oj), rho_bar, hd, SC);
         CPPHF_LAUNCH_CHECK("hartree/contact");
         if (slh) CPPHF_TRY(sl_hartree(K->sl, rho_bar, SC, K->has_contact, W + L.off_slh, st));
     } else if (hd_out) {
