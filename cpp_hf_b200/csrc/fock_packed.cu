@@ -274,10 +274,20 @@ __device__ double kindep_energy(const FusedOut& o, int nb) {
 
 // pass C: rows inverse of the packed channels with the Fock assembly and the
 // energy fused in.  Tile t -> (kx = t / nchunk, chunk q).
-template <class Cx, int N1, int N2>
-__global__ void __launch_bounds__(kPackMaxThreads, 2)
+//
+// One stage: the resident CTAs cover each other's loads, and a second stage only takes
+// the room of a third or fourth CTA.  Up to 96 threads the long transforms get 168
+// registers (four CTAs of 96), beyond that 128 (three of 160): the assembly waits on
+// its loads, so there the number of resident warps decides.  Whole builds against two
+// stages and 128 registers throughout, us: nb = 4 at 256 x 256 49.5/54.2, nb = 7 101/119,
+// nb = 8 136/143, nb = 6 at 144 x 144 38.8/40.6, nb = 8 at 192 x 192 82.1/83.5 (168
+// registers there: 85.3).
+constexpr int kInvThreads = 160;       // 16 lanes of ten channels
+constexpr int kInvSmallThreads = 96;
+template <class Cx, int N1, int N2, int kThreads>
+__global__ void __launch_bounds__(kThreads, kThreads <= kInvSmallThreads ? 4 : 3)
     k_rows_inv_fock_pk(const __grid_constant__ CUtensorMap mT, FusedOut o, ExchangeGeom g, PackGeom pg, int ntiles,
-                       double scale, int nst) {
+                       double scale) {
     constexpr int N = N1 * N2;
     constexpr int kLanes = N1 > N2 ? N1 : N2;  // line lanes: blockDim.x = kLanes * CBp
     constexpr int NE = N / kLanes;             // epilogue points per thread (ky = a + kLanes e)
@@ -286,37 +296,27 @@ __global__ void __launch_bounds__(kPackMaxThreads, 2)
     __shared__ double red[32];
     unsigned char* smem_raw = align128(smem_dyn);
     const int CBp = pg.CBp, nb = pg.nb, nb2 = nb * nb;
-    const PipeLayout L = pipe_layout(N, CBp, sizeof(Cx), false, nst);
+    const PipeLayout L = pipe_layout(N, CBp, sizeof(Cx), false, 1);
     Cx* tw = reinterpret_cast<Cx*>(smem_raw + L.tw);
     unsigned long long* bar = reinterpret_cast<unsigned long long*>(smem_raw + L.bar);
     const int c = threadIdx.x % CBp, a = threadIdx.x / CBp;
     build_line_twiddles(tw, N);
     if (threadIdx.x == 0) {
-        for (int b = 0; b < nst; ++b) mbar_init(&bar[b], 1);
+        mbar_init(bar, 1);
         fence_mbar_init();
     }
     __syncthreads();
-    auto issue = [&](int t, int stage) {
-        if (threadIdx.x != 0) return;
-        const int kx = t / pg.nchunk, q = t - kx * pg.nchunk;
-        unsigned char* st = smem_raw + L.stage0 + (size_t)stage * L.stage_bytes;
-        fence_proxy_async_smem();
-        mbar_arrive_expect_tx(&bar[stage], (unsigned)(N * CBp * sizeof(Cx)));
-        tma_load_3d(st, &mT, 2 * q * CBp, 0, kx, &bar[stage]);
-    };
+    Cx* S = reinterpret_cast<Cx*>(smem_raw + L.stage0);
     Kahan e_k;
-    int i = 0;
-    for (int j = 0; j < nst - 1; ++j)
-        if ((int)blockIdx.x + j * (int)gridDim.x < ntiles) issue(blockIdx.x + j * gridDim.x, j);
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++i) {
-        const int stage = i % nst;
-        {
-            const int ahead = t + (nst - 1) * (int)gridDim.x;
-            if (ahead < ntiles) issue(ahead, (i + nst - 1) % nst);
-        }
-        if (!mbar_wait(&bar[stage], (unsigned)((i / nst) & 1), g.err)) return;
-        Cx* S = reinterpret_cast<Cx*>(smem_raw + L.stage0 + (size_t)stage * L.stage_bytes);
+    unsigned phase = 0;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, phase ^= 1u) {
         const int kx = t / pg.nchunk, q = t - kx * pg.nchunk;
+        if (threadIdx.x == 0) {
+            fence_proxy_async_smem();
+            mbar_arrive_expect_tx(bar, (unsigned)(N * CBp * sizeof(Cx)));
+            tma_load_3d(S, &mT, 2 * q * CBp, 0, kx, bar);
+        }
+        if (!mbar_wait(bar, phase, g.err)) return;
         int r1, r2, L1, L2;
         pack_rows(nb, q, r1, r2, L1, L2);
         const bool live = c < L1 + L2;
@@ -439,7 +439,8 @@ struct PackSpec {
         static std::once_flag once;
         std::call_once(once, [] {
             raise_smem(k_rows_fwd_pk<Cx, N1, N2>);
-            raise_smem(k_rows_inv_fock_pk<Cx, N1, N2>);
+            raise_smem(k_rows_inv_fock_pk<Cx, N1, N2, kInvSmallThreads>);
+            raise_smem(k_rows_inv_fock_pk<Cx, N1, N2, kInvThreads>);
         });
     }
     static int lanes() { return N1 > N2 ? N1 : N2; }
@@ -452,10 +453,9 @@ struct PackSpec {
         return std::max(1, std::min(ntiles, per * num_sms()));
     }
     static bool fits(const PackGeom& pg, bool ref) {
-        if (lanes() * pg.CB > kPackMaxThreads || lanes() * pg.CBp > kPackMaxThreads) return false;
+        if (lanes() * pg.CB > kPackMaxThreads || lanes() * pg.CBp > kInvThreads) return false;
         if (rows_pk_layout(N1 * N2, pg.nb, ref, kPackStages).total > kSmemMax) return false;
-        if (pipe_layout(N1 * N2, pg.CBp, sizeof(Cx), false, kPackStages).total > kSmemMax) return false;
-        return true;
+        return pipe_layout(N1 * N2, pg.CBp, sizeof(Cx), false, 1).total <= kSmemMax;
     }
     static int rows_fwd(const double2* P, const double2* refP, Cx* T, const ExchangeGeom& g, const PackGeom& pg,
                         cudaStream_t st) {
@@ -480,14 +480,14 @@ struct PackSpec {
                                 2ull * pg.Ct, (unsigned long long)g.n1, (unsigned long long)g.n0, row,
                                 row * (unsigned long long)g.n1, 2u * (unsigned)pg.CBp, (unsigned)(N1 * N2), 1u))
             return fail(CPPHF_ERR_CUDA, "packed Fock build: tensor map encoding failed");
-        const PipeLayout L = pipe_layout(N1 * N2, pg.CBp, sizeof(Cx), false, kPackStages);
+        const PipeLayout L = pipe_layout(N1 * N2, pg.CBp, sizeof(Cx), false, 1);
         const int threads = lanes() * pg.CBp;
         const int nt = g.n0 * pg.nchunk;
-        const int grid = std::min(pgrid(k_rows_inv_fock_pk<Cx, N1, N2>, threads, L.total, nt), kFockMaxPartials);
+        auto kern = threads <= kInvSmallThreads ? k_rows_inv_fock_pk<Cx, N1, N2, kInvSmallThreads>
+                                                : k_rows_inv_fock_pk<Cx, N1, N2, kInvThreads>;
+        const int grid = std::min(pgrid(kern, threads, L.total, nt), kFockMaxPartials);
         if (o.energy) CPPHF_CUDA(cudaMemsetAsync(o.counter, 0, sizeof(unsigned), st));
-        k_rows_inv_fock_pk<Cx, N1, N2><<<grid, threads, L.total, st>>>(mT, o, g, pg, nt,
-                                                                       -1.0 / ((double)g.n0 * (double)g.n1),
-                                                                       kPackStages);
+        kern<<<grid, threads, L.total, st>>>(mT, o, g, pg, nt, -1.0 / ((double)g.n0 * (double)g.n1));
         CPPHF_LAUNCH_CHECK("packed Fock build: rows inverse + assembly");
         return CPPHF_OK;
     }
