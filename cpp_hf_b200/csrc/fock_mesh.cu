@@ -11,7 +11,7 @@
 // CTAs are persistent; the energy is Kahan-summed per thread and reduced by the
 // last block in a fixed order.
 //
-// Bound by HBM: T, h and P read, F (and Sigma) written, 4.8 fields of nk nb^2 with
+// Bound by HBM: T, h and P read, F (and Sigma) written, 4.5 fields of nk nb^2 with
 // Sigma.  Measured, 144 x 144, nb = 64 (1.36 GB a field): whole build 2150 us, unfused
 // 3920; this pass 1350 us of it (960 at the copy rate).
 #include "common.cuh"
