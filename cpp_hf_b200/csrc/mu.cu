@@ -47,6 +47,7 @@ constexpr int kMuCluster = 8;                         // CTAs of the cluster for
 constexpr int64_t kMuClusterMax = (int64_t)1 << 16;   // eigenvalues handled by one cluster
 constexpr int kBisectLevels = 3;                      // bisection steps per grid barrier
 constexpr int kMuNV = (1 << kBisectLevels) - 1;       // midpoints evaluated per barrier
+constexpr int kMuSums = (kMuNV + 1) / 2;              // pairs that hold a round's sums
 constexpr double kMuWide = 64.0;                      // exact multisection while the bracket exceeds 64 T
 constexpr int kMuWarmMaxIter = 8;                     // Newton rounds from a warm start before the cold path
 constexpr int kMuSlots = 40;                          // slots of a call (rounds before they are cleared and reused)
@@ -108,9 +109,20 @@ __device__ __forceinline__ void band_major(const MuArgs& a, unsigned i, unsigned
 }
 
 // Cluster barrier: every thread of every CTA of the cluster (hardware barrier;
-// release / acquire at cluster scope orders the partials' global stores).
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+// release / acquire at cluster scope orders the stores to the peers' shared memory).
+__device__ __forceinline__ void cluster_arrive() {
+    __syncwarp();  // the aligned forms want the whole warp
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// v to the place that p has in this block, in the shared memory of block `rank` of the cluster
+__device__ __forceinline__ void st_cluster(double2* p, unsigned rank, double2 v) {
+    unsigned at;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(at), "d"(v.x), "d"(v.y) : "memory");
 }
 
 __device__ __forceinline__ double2 ld_slot(const double2* p) {
@@ -127,24 +139,27 @@ __device__ __forceinline__ double full(double x) { return empty(x) ? NAN : x; }
 
 // Sums (or maxima) over all eigenvalues, one round at a time.  CLUSTER = false: a
 // cooperative grid, or a single block; CLUSTER = true: one thread-block cluster
-// (kMuCluster CTAs) with the hardware cluster barrier and partials in global
-// memory, double-buffered by round parity.
+// (kMuCluster CTAs): every block writes its sums into the shared memory of all
+// blocks, double-buffered by round parity, and the hardware cluster barrier stands
+// between the writes and the reads, so this form touches no global scratch.
 template <bool CLUSTER>
 struct MuSync {
     GridBarrier bar;
     double2* slots;  // [nslots][G]
     int nslots, slot, phase, G;
     double (*red)[32 * kMuNV];  // two trees' scratch, used alternately
+    double2* peers;             // cluster form: [2][kMuSums][kMuCluster], the blocks' sums
     int* failed;
     unsigned* err;
     long long limit;
-    __device__ void init(const MuArgs& a, double (*scratch)[32 * kMuNV], int* fail_flag) {
+    __device__ void init(const MuArgs& a, double (*scratch)[32 * kMuNV], double2* peer_sums, int* fail_flag) {
         bar.init(a.sync, a.spin_limit, a.err);
         slots = reinterpret_cast<double2*>(a.slots);
         nslots = a.nslots;
         slot = phase = 0;
         G = gridDim.x;
         red = scratch;
+        peers = peer_sums;
         failed = fail_flag;
         err = a.err;
         limit = a.spin_limit;
@@ -175,19 +190,21 @@ struct MuSync {
         if (G == 1) return true;
         constexpr int NS = (NV + 1) / 2;
         if constexpr (CLUSTER) {
-            // G = kMuCluster <= 32: every warp reads all partials
-            double2* b = slots + (size_t)(slot & 1) * 4 * G;
+            // a round's buffer is written again two rounds later, behind the barrier that
+            // every reader of this round has passed
+            double2* b = peers + (slot & 1) * kMuSums * kMuCluster;
             ++slot;
-            if (threadIdx.x == 0) {
+            if (threadIdx.x < kMuCluster) {
 #pragma unroll
                 for (int u = 0; u < NS; ++u)
-                    __stcg(&b[u * G + blockIdx.x], mk(v[2 * u], 2 * u + 1 < NV ? v[2 * u + 1] : 0.0));
+                    st_cluster(&b[u * kMuCluster + blockIdx.x], threadIdx.x, mk(v[2 * u], 2 * u + 1 < NV ? v[2 * u + 1] : 0.0));
             }
-            cluster_sync_all();
-            const int lane = threadIdx.x & 31;
+            cluster_arrive();
+            cluster_wait();
+            const int lane = threadIdx.x & 31;  // every warp reads all sums
 #pragma unroll
             for (int u = 0; u < NS; ++u) {
-                const double2 x = lane < G ? __ldcg(&b[u * G + lane]) : mk(MAX ? (double)-INFINITY : 0.0, MAX ? (double)-INFINITY : 0.0);
+                const double2 x = lane < kMuCluster ? b[u * kMuCluster + lane] : mk(MAX ? (double)-INFINITY : 0.0, MAX ? (double)-INFINITY : 0.0);
                 v[2 * u] = op<MAX>(x.x);
                 if (2 * u + 1 < NV) v[2 * u + 1] = op<MAX>(x.y);
             }
@@ -239,7 +256,9 @@ struct MuSync {
 template <bool CLUSTER>
 __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
     __shared__ double red[2][32 * kMuNV];
+    __shared__ double2 peers[CLUSTER ? 2 * kMuSums * kMuCluster : 1];
     __shared__ int failed;
+    if (CLUSTER) cluster_arrive();  // waited for below: no block writes to one that has not started
     if (threadIdx.x == 0) {
         failed = 0;  // ordered by the first tree's barrier
         if (!CLUSTER && blockIdx.x == 0 && gridDim.x > 1) {
@@ -250,7 +269,7 @@ __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
         }
     }
     MuSync<CLUSTER> net;
-    net.init(a, red, &failed);
+    net.init(a, red, peers, &failed);
     const int G = gridDim.x;
     const unsigned nb = (unsigned)a.nb;
     const unsigned n = (unsigned)a.n;
@@ -302,6 +321,7 @@ __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
             ends[1] = fmax(ends[1], e);
         }
     }
+    if (CLUSTER) cluster_wait();
     if (!net.template reduce<2, true>(ends)) return give_up();
     const double emin = -ends[0], emax = ends[1];
     const double Tj = fmax(a.T, 1.0e-12);
@@ -569,11 +589,11 @@ int max_coop_grid() {
 
 
 // ---------------------------------------------------------------------------
-// Allocation-free bisection entry point.  Its scratch (grid-barrier words and
-// block partials, the same layout the workspace variant uses) is this
-// file-scope array, sized for the largest cooperative grid the solver ever
-// launches.  Every GPU that loads the library holds it until the process
-// exits; every call shares it.
+// Allocation-free bisection entry point.  The scratch of its cooperative grid
+// (barrier words and slots, the same layout the workspace variant uses) is this
+// file-scope array, sized for the largest grid the solver ever launches.  Every
+// GPU that loads the library holds it until the process exits; every call of more
+// than kMuClusterMax eigenvalues shares it.
 // ---------------------------------------------------------------------------
 constexpr size_t kMuNoAllocScratchBytes = kMuWsBytes;
 static __device__ __align__(256) unsigned char g_mu_noalloc_scratch[kMuNoAllocScratchBytes];

@@ -116,15 +116,16 @@ int cpphf_find_mu_bisection(const double* eps, const double* weights, int64_t nk
  * kernel - so like any entry point it must not be called from a host function
  * queued on a stream.)  Same arguments and
  * result as cpphf_find_mu_bisection minus the workspace: the scratch (grid
- * barrier words and block partials, about 74 KB) is a file-scope device array
+ * barrier words and block partials, 131136 bytes) is a file-scope device array
  * that every GPU loading the library holds until the process exits.  Limit:
  * nk*nb <= CPPHF_MU_NOALLOC_MAX_EIGENVALUES; larger sizes are rejected with
  * CPPHF_ERR_INVALID.  The first call on a device looks up the array's device
  * address (with that device current) and should come before any stream
  * capture; the cached address is not valid across cudaDeviceReset() or a
  * re-created primary context, so do not use this entry point after either.
- * Calls share the array: each call clears the words that must start at zero,
- * and calls that overlap on the GPU race.  Calls no allocating routine. */
+ * Calls of more than 65536 eigenvalues share the array: each sets the words it
+ * uses, and two of them that overlap on the GPU race.  Smaller calls use none of
+ * it and may overlap with any.  Calls no allocating routine. */
 #define CPPHF_MU_NOALLOC_MAX_EIGENVALUES 2147483647LL
 int cpphf_find_mu_bisection_noalloc(const double* eps, const double* weights, int64_t nk, int64_t nb,
                                     double n_e, double T, int maxiter, double* mu_out, void* stream);
