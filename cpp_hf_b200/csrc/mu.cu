@@ -38,10 +38,12 @@ constexpr int kMuMaxGrid = 1024;
 constexpr int kMuCache = 4;                           // eigenvalues a thread keeps in registers across rounds
 // Forms by the number of eigenvalues, each an ordinary launch but the last.
 // Measured (bisection / in-loop Newton, us), one block against one cluster: 24.8 /
-// 14.5 and 22.8 / 16.5 at 1152 eigenvalues, 53 / 29 and 27 / 16.5 at 4608; one
-// cluster against the cooperative grid: 51 / 31 and 53 / 21 at 18432, 62 / 41 and
-// 47 / 34 at 36864, 118 / 78 and 55 / 29 at 73728.  Up to 2^16 the cluster is kept:
-// concurrent solves (a sweep on 16 streams) do not wait for a whole grid of SMs.
+// 14.5 and 22.8 / 16.5 at 1152 eigenvalues, 53 / 29 and 27 / 16.5 at 4608.  One cluster
+// against the cooperative grid, for a solve alone: 43 / 42 and 49 / 21 at 18432, 64 / 54
+// and 50 / 47 at 36864, 107 / 60 and 43 / 27 at 65536; for eight in-loop solves on each
+// of 16 streams, ms: 1.28 and 1.63, 1.40 and 1.85, 1.44 and 1.48.  Solves that run side
+// by side, as a sweep's do, share the SMs in clusters but queue for the whole grid, and
+// lose by it up to 2^16; a solve alone would gain from the grid from 2^14 on.
 constexpr int64_t kMuOneBlockMax = 1024;              // eigenvalues handled by a single CTA
 constexpr int kMuCluster = 8;                         // CTAs of the cluster form (portable cluster size)
 constexpr int64_t kMuClusterMax = (int64_t)1 << 16;   // eigenvalues handled by one cluster
@@ -61,13 +63,18 @@ __device__ __forceinline__ double expit(double x) {
     return e / (1.0 + e);
 }
 
-// (p, p (1 - p)) of p = 1 / (1 + exp(-x)) from one exponential and one
-// reciprocal: as exact as expit (and p (1 - p) without its cancellation), in half
-// the instructions.  A single block keeps the reference's own expressions: small
-// solves that stop on a plateau depend on the last bits of N(mu).
-__device__ __forceinline__ double2 fermi(double x) {
-    const double e = exp(-fabs(x)), r = 1.0 / (1.0 + e), er = e * r;
-    return mk(x >= 0.0 ? r : er, er * r);
+// a / b from y = 1 / b, q = a y and the residual of q, a correction that leaves the
+// rounding of one division (Markstein, IBM J. Res. Dev. 34 (1990) 111).
+__device__ __forceinline__ double quotient(double a, double b, double q, double y) { return fma(fma(-q, b, a), y, q); }
+
+// expit(d / T) of a cluster or a grid: the values of the reference's expressions with
+// one exponential and one reciprocal.  q = d (1 / T) alone has one rounding more, which
+// the exponential multiplies by |q|; a solve that stops on a plateau depends on the
+// last bits of N(mu) and has to meet the same occupations in every form.  (With the
+// divisions themselves an in-loop solve of 294912 eigenvalues takes 39 us, of 65536 75.)
+__device__ __forceinline__ double expit_quotient(double d, double T, double q, double invT) {
+    const double x = quotient(d, T, q, invT), e = exp(-fabs(x)), b = 1.0 + e, y = 1.0 / b;
+    return x >= 0.0 ? y : quotient(e, b, e * y, y);
 }
 
 // Shortcut thresholds on the (approximate) logistic argument x: for x >= 37,
@@ -137,12 +144,13 @@ __device__ __forceinline__ void st_slot(double2* p, double2 v) {
 __device__ __forceinline__ bool empty(double x) { return __double_as_longlong(x) == -1LL; }
 __device__ __forceinline__ double full(double x) { return empty(x) ? NAN : x; }
 
-// Sums (or maxima) over all eigenvalues, one round at a time.  CLUSTER = false: a
-// cooperative grid, or a single block; CLUSTER = true: one thread-block cluster
-// (kMuCluster CTAs): every block writes its sums into the shared memory of all
+// Sums (or maxima) over all eigenvalues, one round at a time, in one block, a
+// cooperative grid, or one thread-block cluster (kMuCluster CTAs): every block writes its sums into the shared memory of all
 // blocks, double-buffered by round parity, and the hardware cluster barrier stands
 // between the writes and the reads, so this form touches no global scratch.
-template <bool CLUSTER>
+enum class MuForm { kOneBlock, kCluster, kGrid };
+
+template <MuForm FORM>
 struct MuSync {
     GridBarrier bar;
     double2* slots;  // [nslots][G]
@@ -187,9 +195,10 @@ struct MuSync {
     template <int NV, bool MAX = false>
     __device__ bool reduce(double (&v)[NV]) {
         tree<NV, MAX>(v);
-        if (G == 1) return true;
         constexpr int NS = (NV + 1) / 2;
-        if constexpr (CLUSTER) {
+        if constexpr (FORM == MuForm::kOneBlock) {
+            return true;
+        } else if constexpr (FORM == MuForm::kCluster) {
             // a round's buffer is written again two rounds later, behind the barrier that
             // every reader of this round has passed
             double2* b = peers + (slot & 1) * kMuSums * kMuCluster;
@@ -253,22 +262,26 @@ struct MuSync {
     }
 };
 
-template <bool CLUSTER>
+// kOneBlock is a form of its own for its arithmetic: it keeps the reference's
+// expressions as they are written, and a choice between the two at run time costs the
+// others 10 to 20 % (in-loop, 294912 eigenvalues: 39 us against 34).
+template <MuForm FORM>
 __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
+    constexpr bool CLUSTER = FORM == MuForm::kCluster, one = FORM == MuForm::kOneBlock;
     __shared__ double red[2][32 * kMuNV];
     __shared__ double2 peers[CLUSTER ? 2 * kMuSums * kMuCluster : 1];
     __shared__ int failed;
     if (CLUSTER) cluster_arrive();  // waited for below: no block writes to one that has not started
     if (threadIdx.x == 0) {
         failed = 0;  // ordered by the first tree's barrier
-        if (!CLUSTER && blockIdx.x == 0 && gridDim.x > 1) {
+        if (FORM == MuForm::kGrid && blockIdx.x == 0) {
             // barrier words (the launch filled them with the empty pattern): visible before
             // this block's first sums, without which no block comes to use them
             a.sync[0] = a.sync[1] = a.sync[2] = 0u;
             __threadfence();
         }
     }
-    MuSync<CLUSTER> net;
+    MuSync<FORM> net;
     net.init(a, red, peers, &failed);
     const int G = gridDim.x;
     const unsigned nb = (unsigned)a.nb;
@@ -389,7 +402,7 @@ __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
                         if (xa >= kFdOne)
                             v[j] += wk;
                         else if (xa > kFdZero)
-                            v[j] += wk * (G == 1 ? expit(-(e - mid[j]) / Tfd) : fermi(xa).x);
+                            v[j] += wk * (one ? expit((mid[j] - e) / Tfd) : expit_quotient(mid[j] - e, Tfd, xa, invTfd));
                     }
                 }
             });
@@ -426,15 +439,9 @@ __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
                 if (xa >= kFdOne) {
                     v[0] += wk;
                 } else if (xa > kFdZero) {
-                    if (G == 1) {
-                        const double pf = expit(-(e - m) / Tfd);
-                        v[0] += wk * pf;
-                        v[1] += wk * pf * (1.0 - pf) * invTfd;
-                    } else {
-                        const double2 f = fermi(xa);
-                        v[0] += wk * f.x;
-                        v[1] += wk * f.y * invTfd;
-                    }
+                    const double pf = one ? expit((m - e) / Tfd) : expit_quotient(m - e, Tfd, xa, invTfd);
+                    v[0] += wk * pf;
+                    v[1] += wk * pf * (1.0 - pf) * invTfd;
                 }
             });
             if (!net.template reduce<2>(v)) {
@@ -536,19 +543,14 @@ __global__ void __launch_bounds__(kMuThreads) k_mu(MuArgs a) {
                 if (xa >= kFdOne) {
                     v[0] += wk;
                 } else if (xa > kFdZero) {
-                    if (G == 1) {
-                        const double p = expit((mu - e) / Tj);
-                        v[0] += wk * p;
-                        v[1] += wk * p * (1.0 - p) / Tj;
-                    } else {
-                        const double2 f = fermi(xa);
-                        v[0] += wk * f.x;
-                        v[1] += wk * f.y * invTj;
-                    }
+                    const double p = one ? expit((mu - e) / Tj) : expit_quotient(mu - e, Tj, xa, invTj);
+                    const double pq = wk * p * (1.0 - p);
+                    v[0] += wk * p;
+                    v[1] += one ? pq / Tj : pq;  // the reference's terms, or its sum divided once
                 }
             });
             if (!net.template reduce<2>(v)) return give_up();
-            const double N = v[0], Z = v[1];
+            const double N = v[0], Z = one ? v[1] : v[1] / Tj;
             const double mu0 = mu, lo0 = lo, hi0 = hi;
             const double g = N - a.target;
             if (g < 0.0) lo = mu;
@@ -580,7 +582,7 @@ int max_coop_grid() {
     static std::once_flag once;
     std::call_once(once, [] {
         int per = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mu<false>, kMuThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mu<MuForm::kGrid>, kMuThreads, 0);
         if (per < 1) per = 1;
         g = std::min(kMuMaxGrid, per * num_sms());
     });
@@ -634,7 +636,7 @@ int mu_solve(const double* eps, const double* w, int64_t nk, int64_t nb, double 
     a.slots = reinterpret_cast<double*>(static_cast<unsigned char*>(ws) + 64);
     a.nslots = 0;
     if (grid == 1) {
-        k_mu<false><<<1, kMuThreads, 0, st>>>(a);
+        k_mu<MuForm::kOneBlock><<<1, kMuThreads, 0, st>>>(a);
         CPPHF_LAUNCH_CHECK("mu (one block)");
         return CPPHF_OK;
     }
@@ -653,13 +655,13 @@ int mu_solve(const double* eps, const double* w, int64_t nk, int64_t nb, double 
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        CPPHF_CUDA(cudaLaunchKernelEx(&cfg, k_mu<true>, a));
+        CPPHF_CUDA(cudaLaunchKernelEx(&cfg, k_mu<MuForm::kCluster>, a));
         return CPPHF_OK;
     }
     a.nslots = (int)std::min<int64_t>(kMuSlots, (int64_t)(kMuWsBytes - 64) / 16 / grid);
     CPPHF_CUDA(cudaMemsetAsync(ws, 0xFF, 64 + 16 * (size_t)a.nslots * grid, st));
     void* args[] = {&a};
-    CPPHF_CUDA(cudaLaunchCooperativeKernel((const void*)k_mu<false>, dim3(grid), dim3(kMuThreads), args, 0, st));
+    CPPHF_CUDA(cudaLaunchCooperativeKernel((const void*)k_mu<MuForm::kGrid>, dim3(grid), dim3(kMuThreads), args, 0, st));
     return CPPHF_OK;
 }
 
