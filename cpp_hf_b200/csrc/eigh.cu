@@ -73,6 +73,7 @@ int eigh_batched(const double2* M, double* w, double2* V, int64_t batch, int64_t
         for (int i = 0; i < nb; ++i) bs.blk[i] = 0;
     }
     if (bs.nblocks <= 1 && eigh_small_enabled(nb)) return eigh_small(M, w, V, batch, nb, mode, st);
+    if (eigh_blocks_enabled(batch, bs)) return eigh_blocks(M, w, V, batch, nb, mode, bs, st);
     return eigh_dc(M, w, V, batch, nb, mode, bs, st);
 }
 

@@ -26,10 +26,14 @@ int make_block_spec(int64_t nb, const int64_t* sizes, int64_t n_sizes, int sort,
 int block_structure_ok(const double2* M, int64_t batch, int64_t nb, const BlockSpec& bs, unsigned long long* dev2,
                        cudaStream_t st, bool* ok);
 
-// Householder + implicit QL for 2 <= nb <= 8 (eigh_small.cu: a thread or
-// eight lanes per matrix); other nb, and block structures, run eigh_dc.
+// Householder + implicit QL for nb <= 8 (eigh_small.cu: a thread or eight lanes
+// per matrix); block structures of small blocks take them block by block
+// (eigh_blocks), everything else runs eigh_dc.
 bool eigh_small_enabled(int64_t nb);
 int eigh_small(const double2* M, double* w, double2* V, int64_t batch, int64_t nb, int mode, cudaStream_t st);
+bool eigh_blocks_enabled(int64_t batch, const BlockSpec& bs);
+int eigh_blocks(const double2* M, double* w, double2* V, int64_t batch, int64_t nb, int mode, const BlockSpec& bs,
+                cudaStream_t st);
 
 // Householder + divide and conquer (eigh_dc.cu: one CTA per matrix), any nb <= kMaxEighNb
 int eigh_dc(const double2* M, double* w, double2* V, int64_t batch, int64_t nb, int mode, const BlockSpec& bs,

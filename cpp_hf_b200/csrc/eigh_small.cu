@@ -26,6 +26,7 @@
 #include "common.cuh"
 #include "eigh.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 #include <mutex>
 
@@ -365,11 +366,34 @@ struct ThreadGeo {
     static constexpr size_t kSmem = sizeof(double) * WORDS * kThreadCta + sizeof(double2) * STG * kThreadCta;
 };
 
-template <int NB>
+// The diagonal blocks of one size of a batch of ld x ld matrices: problem k is block
+// k % count of matrix k / count.
+struct BlockClass {
+    int ld, count;
+    short start[kMaxEighNb];
+};
+
+// BLOCKS: the matrices are the diagonal blocks bc, and eigenvalues and vectors go to
+// the places of the block (k_block_order then finishes V); a block with a NaN or an
+// infinity gives NaN, as eigh_dc does.
+template <int NB, bool BLOCKS>
 __global__ void __launch_bounds__(kThreadCta, 4)
     k_eigh_thread(const double2* __restrict__ M, double* __restrict__ w, double2* __restrict__ Vout, int64_t batch,
-                  int mode) {
+                  int mode, const __grid_constant__ BlockClass bc) {
     using G = ThreadGeo<NB>;
+    constexpr bool kNanOut = BLOCKS || NB == 1;
+    const int ld = BLOCKS ? bc.ld : NB;
+    // element (0, 0) of problem p, and its first eigenvalue
+    auto origin = [&](int64_t p) -> size_t {
+        if (!BLOCKS) return (size_t)p * NB * NB;
+        const int64_t m = p / bc.count;
+        return (size_t)m * ld * ld + (size_t)bc.start[p - m * bc.count] * (ld + 1);
+    };
+    auto first = [&](int64_t p) -> size_t {
+        if (!BLOCKS) return (size_t)p * NB;
+        const int64_t m = p / bc.count;
+        return (size_t)m * ld + bc.start[p - m * bc.count];
+    };
     extern __shared__ __align__(16) unsigned char raw[];
     double* sm = reinterpret_cast<double*>(raw) + threadIdx.x;  // word i of the thread at sm[i * kThreadCta]
     const int lane = threadIdx.x & 31, wbase = threadIdx.x - lane;
@@ -385,17 +409,18 @@ __global__ void __launch_bounds__(kThreadCta, 4)
     constexpr auto uoff = [](int kk) { return kk * (NB - 1) - kk * (kk - 1) / 2 - (kk + 1); };  // entry of u_kk[i]: + i
 
     double d[NB], e[NB];
+    double nan = 0.0;  // 0, or NaN once an entry is not finite
     int ex = 0;
     {
         // lower triangle of herm(M) or herm(i M), scaled by a power of two
         double2 a[NB][NB];
-        const double2* Mk = M + (size_t)k * NB * NB;
+        const double2* Mk = M + origin(k);
         double amax = 0.0;
 #pragma unroll
         for (int i = 0; i < NB; ++i)
 #pragma unroll
             for (int j = 0; j < NB; ++j) {
-                double2 x = Mk[i * NB + j];
+                double2 x = Mk[i * ld + j];
                 if (mode == 1) x = mk(-x.y, x.x);
                 if (j < i) {
                     a[i][j] = x;  // finished when row j's entry (j, i) was read before
@@ -408,7 +433,10 @@ __global__ void __launch_bounds__(kThreadCta, 4)
         for (int i = 0; i < NB; ++i) {
             a[i][i].y = 0.0;
 #pragma unroll
-            for (int j = 0; j <= i; ++j) amax = fmax(amax, fmax(fabs(a[i][j].x), fabs(a[i][j].y)));
+            for (int j = 0; j <= i; ++j) {
+                amax = fmax(amax, fmax(fabs(a[i][j].x), fabs(a[i][j].y)));
+                if (kNanOut) nan += 0.0 * a[i][j].x + 0.0 * a[i][j].y;
+            }
         }
         if (amax > 0.0 && isfinite(amax)) frexp(amax, &ex);
         const double sc = ldexp(1.0, -ex);
@@ -571,7 +599,7 @@ __global__ void __launch_bounds__(kThreadCta, 4)
     const int cnt = (int)min((int64_t)32, batch - k0);
     if (lane < cnt) {
 #pragma unroll
-        for (int i = 0; i < NB; ++i) w[(size_t)k * NB + i] = ldexp(d[i], ex);
+        for (int i = 0; i < NB; ++i) w[first(k) + i] = ldexp(d[i], ex) + nan;
     }
     // ---- 5. V = H_0 .. H_{NB-3} diag(delta) Z, two columns at a time ----
 #pragma unroll
@@ -607,28 +635,103 @@ __global__ void __launch_bounds__(kThreadCta, 4)
 #pragma unroll
         for (int i = 0; i < NB; ++i)
 #pragma unroll
-            for (int c = 0; c < W; ++c) stg[lane * G::STG + 2 * i + c] = v[c][i];
+            for (int c = 0; c < W; ++c) stg[lane * G::STG + 2 * i + c] = kNanOut ? mk(v[c][i].x + nan, v[c][i].y + nan) : v[c][i];
         __syncwarp();
         for (int x = lane; x < cnt * NB * W; x += 32) {
             const int mat = x / (NB * W), r = x - mat * (NB * W), i = r / W, c = r - i * W;
-            if (c < nc) Vout[((size_t)(k0 + mat) * NB + i) * NB + c0 + c] = stg[mat * G::STG + r];
+            if (c < nc) Vout[origin(k0 + mat) + (size_t)i * ld + c0 + c] = stg[mat * G::STG + r];
         }
     }
 }
 
-template <int NB>
-int launch_thread(const double2* M, double* w, double2* V, int64_t batch, int mode, cudaStream_t st) {
+template <int NB, bool BLOCKS>
+int launch_thread(const double2* M, double* w, double2* V, int64_t batch, int mode, const BlockClass& bc, cudaStream_t st) {
     static std::once_flag once;
-    std::call_once(once, [] { raise_smem(k_eigh_thread<NB>); });
+    std::call_once(once, [] { raise_smem(k_eigh_thread<NB, BLOCKS>); });
     const unsigned grid = (unsigned)((batch + kThreadCta - 1) / kThreadCta);
-    k_eigh_thread<NB><<<grid, kThreadCta, ThreadGeo<NB>::kSmem, st>>>(M, w, V, batch, mode);
+    k_eigh_thread<NB, BLOCKS><<<grid, kThreadCta, ThreadGeo<NB>::kSmem, st>>>(M, w, V, batch, mode, bc);
     CPPHF_LAUNCH_CHECK("eigh (thread per matrix)");
     return CPPHF_OK;
 }
 
+template <bool BLOCKS>
+int thread_per_matrix(int nb, const double2* M, double* w, double2* V, int64_t batch, int mode, const BlockClass& bc,
+                      cudaStream_t st) {
+    switch (nb) {
+        case 1: return launch_thread<1, BLOCKS>(M, w, V, batch, mode, bc, st);
+        case 2: return launch_thread<2, BLOCKS>(M, w, V, batch, mode, bc, st);
+        case 3: return launch_thread<3, BLOCKS>(M, w, V, batch, mode, bc, st);
+        case 4: return launch_thread<4, BLOCKS>(M, w, V, batch, mode, bc, st);
+        case 5: return launch_thread<5, BLOCKS>(M, w, V, batch, mode, bc, st);
+        case 6: return launch_thread<6, BLOCKS>(M, w, V, batch, mode, bc, st);
+        case 7: return launch_thread<7, BLOCKS>(M, w, V, batch, mode, bc, st);
+        case 8: return launch_thread<8, BLOCKS>(M, w, V, batch, mode, bc, st);
+        default: break;
+    }
+    return fail(CPPHF_ERR_UNSUPPORTED, "small-matrix eigensolver called with unsupported nb");
+}
+
+// A total order of the doubles (NaN included), so that the ranks are a permutation.
+__device__ __forceinline__ unsigned long long order_key(double x) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    return (b >> 63) ? ~b : b | 0x8000000000000000ull;
+}
+
+// After the blocks of every size: zeros outside the blocks, and with sort the
+// eigenvalues ascending over the whole matrix (stable), in place.  A matrix with a
+// NaN among its eigenvalues becomes NaN.  Bound by HBM (V read and written once); a CTA
+// holds tiles of whole matrices, about kOrderTile entries, in shared memory.
+constexpr int kOrderTile = 1024;
+constexpr int kOrderThreads = 256;
+__host__ __device__ constexpr int order_matrices(int nb) { return nb * nb >= kOrderTile ? 1 : kOrderTile / (nb * nb); }
+
+__global__ void __launch_bounds__(kOrderThreads)
+    k_block_order(double* __restrict__ w, double2* __restrict__ V, int64_t batch, int nb, const __grid_constant__ BlockSpec bs) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    const int nb2 = nb * nb, KT = order_matrices(nb);
+    const int64_t k0 = (int64_t)blockIdx.x * KT;
+    const int cnt = (int)min((int64_t)KT, batch - k0);
+    double2* T = reinterpret_cast<double2*>(raw);
+    double* ws = reinterpret_cast<double*>(T + (size_t)KT * nb2);
+    int* from = reinterpret_cast<int*>(ws + (size_t)KT * nb);
+    int* nan = from + (size_t)KT * nb;
+    double2* Vk = V + (size_t)k0 * nb2;
+    double* wk = w + (size_t)k0 * nb;
+    for (int e = threadIdx.x; e < cnt * nb2; e += kOrderThreads) {
+        const int r = e % nb2, i = r / nb, j = r - i * nb;
+        T[e] = bs.blk[i] == bs.blk[j] ? Vk[e] : mk(0.0, 0.0);
+    }
+    for (int e = threadIdx.x; e < cnt; e += kOrderThreads) nan[e] = 0;
+    __syncthreads();
+    for (int e = threadIdx.x; e < cnt * nb; e += kOrderThreads) {
+        ws[e] = wk[e];
+        if (isnan(ws[e])) nan[e / nb] = 1;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < cnt * nb; e += kOrderThreads) {
+        const int m = e / nb, j = e - m * nb;
+        int rank = j;
+        if (bs.sort) {
+            const unsigned long long kj = order_key(ws[e]);
+            rank = 0;
+            for (int i = 0; i < nb; ++i) {
+                const unsigned long long ki = order_key(ws[m * nb + i]);
+                rank += ki < kj || (ki == kj && i < j) ? 1 : 0;
+            }
+        }
+        from[m * nb + rank] = j;
+        wk[m * nb + rank] = nan[m] ? NAN : ws[e];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < cnt * nb2; e += kOrderThreads) {
+        const int m = e / nb2, r = e - m * nb2, i = r / nb, j = r - i * nb;
+        Vk[e] = nan[m] ? mk((double)NAN, (double)NAN) : T[m * nb2 + i * nb + from[m * nb + j]];
+    }
+}
+
 }  // namespace
 
-bool eigh_small_enabled(int64_t nb) { return nb >= 2 && nb <= 8; }
+bool eigh_small_enabled(int64_t nb) { return nb >= 1 && nb <= 8; }
 
 int eigh_small(const double2* M, double* w, double2* V, int64_t batch, int64_t nb, int mode, cudaStream_t st) {
     // A thread's chain takes 2.6 (nb = 2) to 55 us (nb = 8) however small the batch,
@@ -638,18 +741,7 @@ int eigh_small(const double2* M, double* w, double2* V, int64_t batch, int64_t n
     // at 36864; nb = 6 23.5 / 22.4 at 4608, 23.6 / 25.6 at 6912, 32.7 / 114 at 36864;
     // nb = 8 53.4 / 42.5 at 6912, 52.7 / 53.2 at 9216, 81.4 / 249 at 36864.
     const int64_t least = nb <= 4 ? 0 : nb <= 6 ? 5632 : 9216;
-    if (batch >= least) {
-        switch (nb) {
-            case 2: return launch_thread<2>(M, w, V, batch, mode, st);
-            case 3: return launch_thread<3>(M, w, V, batch, mode, st);
-            case 4: return launch_thread<4>(M, w, V, batch, mode, st);
-            case 5: return launch_thread<5>(M, w, V, batch, mode, st);
-            case 6: return launch_thread<6>(M, w, V, batch, mode, st);
-            case 7: return launch_thread<7>(M, w, V, batch, mode, st);
-            case 8: return launch_thread<8>(M, w, V, batch, mode, st);
-            default: break;
-        }
-    }
+    if (batch >= least) return thread_per_matrix<false>((int)nb, M, w, V, batch, mode, BlockClass(), st);
     const unsigned grid = (unsigned)((batch * kGroup + kHqlThreads - 1) / kHqlThreads);
     switch (nb) {
         case 5: k_eigh_hql<5><<<grid, kHqlThreads, 0, st>>>(M, w, V, batch, mode); break;
@@ -659,6 +751,39 @@ int eigh_small(const double2* M, double* w, double2* V, int64_t batch, int64_t n
         default: return fail(CPPHF_ERR_UNSUPPORTED, "eigh_small: nb out of range");
     }
     CPPHF_LAUNCH_CHECK("eigh (Householder + QL)");
+    return CPPHF_OK;
+}
+
+// Block by block where every block has a thread kernel.  Measured against eigh_dc on
+// whole matrices and the cyclic Jacobi kernel before it (us): 36864 matrices of nb = 8,
+// blocks of 2: 28 / 587 / 152, of 4: 51 / 896 / 637; of nb = 4, blocks of 2: 16 / 360 / 76;
+// 5184 of nb = 64, blocks of 8: 450 / 3843 / 38900.  A thread's chain for a block of 7
+// or 8 is longer than eigh_dc's for up to 16 rows, while that takes one wave (12
+// CTAs per SM): 1296 matrices of two blocks of 8 76 / 68, but 5184 80 / 212.
+bool eigh_blocks_enabled(int64_t batch, const BlockSpec& bs) {
+    if (bs.nblocks <= 1) return false;
+    int largest = 0;
+    for (int b = 0; b < bs.nblocks; ++b) largest = std::max(largest, bs.start[b + 1] - bs.start[b]);
+    if (largest >= 7 && bs.start[bs.nblocks] <= 16 && batch <= 12 * (int64_t)num_sms()) return false;
+    return largest <= 8;
+}
+
+int eigh_blocks(const double2* M, double* w, double2* V, int64_t batch, int64_t nb, int mode, const BlockSpec& bs,
+                cudaStream_t st) {
+    for (int size = 1; size <= 8; ++size) {
+        BlockClass bc;
+        bc.ld = (int)nb;
+        bc.count = 0;
+        for (int b = 0; b < bs.nblocks; ++b)
+            if (bs.start[b + 1] - bs.start[b] == size) bc.start[bc.count++] = bs.start[b];
+        if (bc.count) CPPHF_TRY(thread_per_matrix<true>(size, M, w, V, batch * bc.count, mode, bc, st));
+    }
+    static std::once_flag once;
+    std::call_once(once, [] { raise_smem(k_block_order); });
+    const size_t KT = (size_t)order_matrices((int)nb);
+    const size_t smem = KT * (sizeof(double2) * nb * nb + (sizeof(double) + sizeof(int)) * nb + sizeof(int));
+    k_block_order<<<(unsigned)((batch + KT - 1) / KT), kOrderThreads, smem, st>>>(w, V, batch, (int)nb, bs);
+    CPPHF_LAUNCH_CHECK("eigh (order of the blocks)");
     return CPPHF_OK;
 }
 
