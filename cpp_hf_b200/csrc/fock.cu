@@ -42,7 +42,7 @@ constexpr int kTileElems = 1024;  // k-blocks of at most this many elements take
 // Bound by HBM for large meshes (P and refP read once), by the chain of the two
 // tickets for small ones.  Whole builds with refP and two contact terms, us, against
 // 256-thread partials summed serially by a second, single-block kernel: 192 x 192,
-// nb = 8: 127/159; 75 x 98, nb = 5: 61/74; 48 x 48, nb = 2: 42/45; 36 x 36, nb = 64:
+// nb = 8: 127/159; 75 x 98, nb = 5: 61/74; 48 x 48, nb = 2: 37/42; 36 x 36, nb = 64:
 // 399/6575 (the products there were formed entry by entry, nb^4).
 constexpr int kRhoThreads = 1024;
 constexpr int kRhoChannels = 256;
@@ -62,6 +62,19 @@ __global__ void __launch_bounds__(kRhoThreads)
     const bool live = lane < lanes && c < nb2;
     const int64_t per = (nk + Gk - 1) / Gk, k0 = blockIdx.x * per, k1 = min(nk, k0 + per);
     double2 acc = mk(0.0, 0.0);
+    // acc of lane 0 <- the channel's sum over the lanes: a tree, since one or two bands
+    // leave 1024 or 256 lanes to a channel (one band at 192 x 192, whole build: 46 us, with
+    // the lanes added one by one 68)
+    auto lane_sum = [&]() {
+        acc_sh[tid] = acc;
+        for (int s = 1 << (31 - __clz(lanes - 1)); s > 0; s >>= 1) {
+            __syncthreads();
+            if (live && lane < s && lane + s < lanes) {
+                acc = cadd(acc, acc_sh[(lane + s) * CH + cl]);
+                acc_sh[tid] = acc;
+            }
+        }
+    };
     if (live) {
         int64_t k = k0 + lane;
         for (; k + 3 * lanes < k1; k += 4 * lanes) {
@@ -88,10 +101,8 @@ __global__ void __launch_bounds__(kRhoThreads)
             acc.y += w[k] * v.y;
         }
     }
-    acc_sh[tid] = acc;
-    __syncthreads();
+    lane_sum();
     if (lane == 0 && live) {
-        for (int l = 1; l < lanes; ++l) acc = cadd(acc, acc_sh[l * CH + cl]);
         st_l2(part + (size_t)blockIdx.x * nb2 + c, acc);
         __threadfence();
     }
@@ -105,10 +116,8 @@ __global__ void __launch_bounds__(kRhoThreads)
 #pragma unroll 4
         for (int b = lane; b < Gk; b += lanes) acc = cadd(acc, ld_l2(part + (size_t)b * nb2 + c));
     }
-    acc_sh[tid] = acc;
-    __syncthreads();
+    lane_sum();
     if (lane == 0 && live) {
-        for (int l = 1; l < lanes; ++l) acc = cadd(acc, acc_sh[l * CH + cl]);
         st_l2(rho_bar + c, acc);
         __threadfence();
     }
