@@ -18,8 +18,9 @@
 // 24, 32, 36, 48, 64, 72, 96, 128, 144, 192, 256, 288) run the four-step
 // transform with global loads/stores straight from/to registers and one
 // shared-memory transpose per direction; other lengths run the mixed-radix passes
-// of exchange_smooth.cu in complex128 (also for zero-padded fields) and the
-// out-of-place Stockham stages of fft.cuh in complex64.
+// of exchange_smooth.cu in complex128 (also for zero-padded fields), and the
+// out-of-place Stockham stages of fft.cuh in complex64 and in the complex128 passes
+// too small to fill the chip (smooth_pays).
 #include "common.cuh"
 #include "exchange.cuh"
 #include "fft.cuh"
@@ -867,19 +868,18 @@ int pass_rows_fwd(const double2* P, const double2* refP, Cx* T, const ExchangeGe
         default: break;
     }
     if constexpr (std::is_same_v<Cx, double2>) {
-        return smooth_rows_fwd(P, refP, T, g, st);
-    } else {
-        FftPlan1D pl;
-        if (!make_plan(g.n1, pl)) return fail(CPPHF_ERR_INVALID, "exchange: mesh size has too many prime factors");
-        Gen<Cx>::attrs();
-        const Launch L = plan_launch(g.n1, g.C, sizeof(Cx), g.n1, true);
-        if (L.smem > kSmemMax)
-            return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
-        k_rows_fwd_g<Cx><<<dim3(g.n0, L.nchunk), cap_threads(k_rows_fwd_g<Cx>, L.threads), L.smem, st>>>(P, refP, T, g,
-                                                                                                         pl, L.CB);
-        CPPHF_LAUNCH_CHECK("exchange rows forward");
-        return CPPHF_OK;
+        if (smooth_pays(g.n1, (int64_t)g.n0 * g.n1 * g.C, false)) return smooth_rows_fwd(P, refP, T, g, st);
     }
+    FftPlan1D pl;
+    if (!make_plan(g.n1, pl)) return fail(CPPHF_ERR_INVALID, "exchange: mesh size has too many prime factors");
+    Gen<Cx>::attrs();
+    const Launch L = plan_launch(g.n1, g.C, sizeof(Cx), g.n1, true);
+    if (L.smem > kSmemMax)
+        return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
+    k_rows_fwd_g<Cx><<<dim3(g.n0, L.nchunk), cap_threads(k_rows_fwd_g<Cx>, L.threads), L.smem, st>>>(P, refP, T, g,
+                                                                                                     pl, L.CB);
+    CPPHF_LAUNCH_CHECK("exchange rows forward");
+    return CPPHF_OK;
 }
 
 template <class Cx>
@@ -892,19 +892,18 @@ int pass_cols(Cx* T, const double2* VR, const ExchangeGeom& g, int vmode, cudaSt
         default: break;
     }
     if constexpr (std::is_same_v<Cx, double2>) {
-        return smooth_cols(T, VR, g, vmode, st);
-    } else {
-        FftPlan1D pl;
-        if (!make_plan(g.n0, pl)) return fail(CPPHF_ERR_INVALID, "exchange: mesh size has too many prime factors");
-        Gen<Cx>::attrs();
-        const Launch L = plan_launch(g.n0, g.C, sizeof(Cx), g.n0, true);
-        if (L.smem > kSmemMax)
-            return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
-        k_cols_conv_g<Cx><<<dim3(g.n1, L.nchunk), cap_threads(k_cols_conv_g<Cx>, L.threads), L.smem, st>>>(T, VR, g, pl,
-                                                                                                           L.CB, vmode);
-        CPPHF_LAUNCH_CHECK("exchange columns convolve");
-        return CPPHF_OK;
+        if (smooth_pays(g.n0, (int64_t)g.n0 * g.n1 * g.C, true)) return smooth_cols(T, VR, g, vmode, st);
     }
+    FftPlan1D pl;
+    if (!make_plan(g.n0, pl)) return fail(CPPHF_ERR_INVALID, "exchange: mesh size has too many prime factors");
+    Gen<Cx>::attrs();
+    const Launch L = plan_launch(g.n0, g.C, sizeof(Cx), g.n0, true);
+    if (L.smem > kSmemMax)
+        return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
+    k_cols_conv_g<Cx><<<dim3(g.n1, L.nchunk), cap_threads(k_cols_conv_g<Cx>, L.threads), L.smem, st>>>(T, VR, g, pl,
+                                                                                                       L.CB, vmode);
+    CPPHF_LAUNCH_CHECK("exchange columns convolve");
+    return CPPHF_OK;
 }
 
 template <class Cx>
@@ -917,19 +916,18 @@ int pass_rows_inv(const Cx* T, double2* Sigma, const ExchangeGeom& g, double sca
         default: break;
     }
     if constexpr (std::is_same_v<Cx, double2>) {
-        return smooth_rows_inv(T, Sigma, g, scale, st);
-    } else {
-        FftPlan1D pl;
-        if (!make_plan(g.n1, pl)) return fail(CPPHF_ERR_INVALID, "exchange: mesh size has too many prime factors");
-        Gen<Cx>::attrs();
-        const Launch L = plan_launch(g.n1, g.C, sizeof(Cx), g.n1, true);
-        if (L.smem > kSmemMax)
-            return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
-        k_rows_inv_g<Cx><<<dim3(g.n0, L.nchunk), cap_threads(k_rows_inv_g<Cx>, L.threads), L.smem, st>>>(T, Sigma, g, pl,
-                                                                                                         L.CB, scale);
-        CPPHF_LAUNCH_CHECK("exchange rows inverse");
-        return CPPHF_OK;
+        if (smooth_pays(g.n1, (int64_t)g.n0 * g.n1 * g.C, false)) return smooth_rows_inv(T, Sigma, g, scale, st);
     }
+    FftPlan1D pl;
+    if (!make_plan(g.n1, pl)) return fail(CPPHF_ERR_INVALID, "exchange: mesh size has too many prime factors");
+    Gen<Cx>::attrs();
+    const Launch L = plan_launch(g.n1, g.C, sizeof(Cx), g.n1, true);
+    if (L.smem > kSmemMax)
+        return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
+    k_rows_inv_g<Cx><<<dim3(g.n0, L.nchunk), cap_threads(k_rows_inv_g<Cx>, L.threads), L.smem, st>>>(T, Sigma, g, pl,
+                                                                                                     L.CB, scale);
+    CPPHF_LAUNCH_CHECK("exchange rows inverse");
+    return CPPHF_OK;
 }
 
 template <class Cx>

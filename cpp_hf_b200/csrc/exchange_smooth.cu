@@ -534,10 +534,15 @@ struct SmoothLaunch {
 };
 
 // channels per tile: about kSmoothTile points (so that two to three CTAs fit an
-// SM), in balanced chunks
-SmoothLaunch smooth_launch(int n, int C) {
+// SM), fewer (down to four, a 64-byte run) where the pass would have a tile for less than
+// three SMs in five, in balanced chunks: 37 x 37, nb = 8 24.2 -> 19.8 us an exchange,
+// 19 x 19, nb = 16 29.7 -> 18.1; a tile for every SM instead took 26.9 -> 32.9 at
+// 31 x 31, nb = 16
+SmoothLaunch smooth_launch(int n, int C, int lines) {
     SmoothLaunch L;
-    const int cap = std::max(1, std::min({C, kSmoothTile / n, kSmoothThreads}));
+    const int64_t tiles = std::max(1, 3 * num_sms() / 5);
+    const int per_sm = (int)std::min<int64_t>(C, ((int64_t)lines * C + tiles - 1) / tiles);
+    const int cap = std::max(1, std::min({C, kSmoothTile / n, kSmoothThreads, std::max(per_sm, 4)}));
     const int nch = (C + cap - 1) / cap;
     L.CB = (C + nch - 1) / nch;
     L.nchunk = (C + L.CB - 1) / L.CB;
@@ -563,9 +568,9 @@ void smooth_attrs() {
     });
 }
 
-bool ready(int n, int C, SmoothPlan& pl, SmoothLaunch& L) {
+bool ready(int n, int C, int lines, SmoothPlan& pl, SmoothLaunch& L) {
     if (!smooth_plan(n, pl)) return false;
-    L = smooth_launch(n, C);
+    L = smooth_launch(n, C, lines);
     if (L.smem > kSmemMax) return false;
     smooth_attrs();
     return true;
@@ -573,15 +578,37 @@ bool ready(int n, int C, SmoothPlan& pl, SmoothLaunch& L) {
 
 }  // namespace
 
+// Small passes wait for the chain of one butterfly, which grows with the radix; the
+// Stockham stages of fft.cuh, an output per thread, have the shorter one and lose once
+// their R loads and FMAs per point fill the SMs.  Measured in whole exchanges, both row
+// passes / the columns pass here less there, us: n = 100 +3.7 / -0.6 up to 2^12 points
+// (n x lines x channels), +1.3 / -1.9 in [2^15, 2^16), -2.4 / -5.9 beyond; n = 13 +2.4 /
+// +1.2, +1.3 / +0.6, -0.6 / -0.8; n = 21 +0.7 / -1.0, -1.0 / -2.1; n = 75 +3.3 / +0.8,
+// +1.1 / -0.6; n = 19 (a direct sum) +0.5 / +0.4 up to 2^13, +0.2 / +0.2, -2.8 / -2.4.
+// Longer primes (47: -0.7 / 0; 251: -7.4 / -2.8) and lines of more than 240 points (384:
+// -2.9 / -5.8) win or tie here at any size.
+bool smooth_pays(int n, int64_t points, bool columns) {
+    constexpr int64_t k14 = 1 << 14, k15 = 1 << 15, k16 = 1 << 16;
+    SmoothPlan pl;
+    if (n > 240 || points >= k16 || !smooth_plan(n, pl)) return true;
+    bool long_odd = n < 16 && n % 2 == 1;  // a single radix of 7, 11, 13 or 15 ends in one here
+    for (int i = 0; i < pl.ns; ++i) {
+        if (pl.r[i] > 16) return n > 37 || points >= k14;
+        long_odd = long_odd || pl.r[i] == 13 || pl.r[i] == 15;
+    }
+    if (columns) return points >= k15 || !long_odd;
+    return points >= (n < 16 || (n >= 96 && n <= 192) ? k16 : k15);
+}
+
 bool smooth_supported(int n, int C) {
     SmoothPlan pl;
-    return smooth_plan(n, pl) && smooth_launch(n, C).smem <= kSmemMax;
+    return smooth_plan(n, pl) && smooth_launch(n, C, 65535).smem <= kSmemMax;
 }
 
 int smooth_rows_fwd(const double2* P, const double2* refP, double2* T, const ExchangeGeom& g, cudaStream_t st) {
     SmoothPlan pl;
     SmoothLaunch L;
-    if (!ready(g.n1, g.C, pl, L)) return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
+    if (!ready(g.n1, g.C, g.s0, pl, L)) return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
     const int nt = g.s0 * L.nchunk;
     k_rows_fwd_m<<<smooth_grid(k_rows_fwd_m, L, nt), L.threads, L.smem, st>>>(P, refP, T, g, pl, L.CB, L.nchunk, nt);
     CPPHF_LAUNCH_CHECK("exchange rows forward");
@@ -591,7 +618,7 @@ int smooth_rows_fwd(const double2* P, const double2* refP, double2* T, const Exc
 int smooth_cols(double2* T, const double2* VR, const ExchangeGeom& g, int vmode, cudaStream_t st) {
     SmoothPlan pl;
     SmoothLaunch L;
-    if (!ready(g.n0, g.C, pl, L)) return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
+    if (!ready(g.n0, g.C, g.n1, pl, L)) return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
     const int nt = g.n1 * L.nchunk;
     k_cols_conv_m<<<smooth_grid(k_cols_conv_m, L, nt), L.threads, L.smem, st>>>(T, VR, g, pl, L.CB, L.nchunk, nt, vmode);
     CPPHF_LAUNCH_CHECK("exchange columns convolve");
@@ -601,7 +628,7 @@ int smooth_cols(double2* T, const double2* VR, const ExchangeGeom& g, int vmode,
 int smooth_rows_inv(const double2* T, double2* Sigma, const ExchangeGeom& g, double scale, cudaStream_t st) {
     SmoothPlan pl;
     SmoothLaunch L;
-    if (!ready(g.n1, g.C, pl, L)) return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
+    if (!ready(g.n1, g.C, g.s0, pl, L)) return fail(CPPHF_ERR_UNSUPPORTED, "exchange: mesh axis too long for the shared-memory FFT");
     const int nt = g.s0 * L.nchunk;
     k_rows_inv_m<<<smooth_grid(k_rows_inv_m, L, nt), L.threads, L.smem, st>>>(T, Sigma, g, pl, L.CB, L.nchunk, nt, scale);
     CPPHF_LAUNCH_CHECK("exchange rows inverse");
