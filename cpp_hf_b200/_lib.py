@@ -118,6 +118,7 @@ _SIGS = {
     "cpphf_solve_mu_inloop": (C.c_int, [vp, vp, i64, i64, f64, vp, f64, C.c_int, vp, vp, sz, vp]),
     "cpphf_find_mu_bisection_noalloc": (C.c_int, [vp, vp, i64, i64, f64, f64, C.c_int, vp, vp]),
     "cpphf_build_fock_workspace_bytes": (sz, [C.POINTER(Kernel)]),
+    "cpphf_build_fock_fused": (C.c_int, [C.POINTER(Kernel)]),
     "cpphf_kernel_packed_bytes": (sz, [C.POINTER(Kernel)]),
     "cpphf_kernel_pack": (C.c_int, [C.POINTER(Kernel), vp, vp, vp]),
     "cpphf_vr_hermitian_deviation": (C.c_int, [vp, i64, i64, i64, vp, vp]),

@@ -581,6 +581,8 @@ int build_fock(const cpphf_kernel* K, const double2* P, double2* Sigma, double2*
 
 extern "C" {
 
+int cpphf_build_fock_fused(const cpphf_kernel* K) { return K ? cpphf::fused_build(K) : 0; }
+
 size_t cpphf_build_fock_workspace_bytes(const cpphf_kernel* K) {
     return K ? cpphf::build_fock_workspace_bytes(K) : 0;
 }

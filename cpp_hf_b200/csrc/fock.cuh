@@ -35,9 +35,9 @@ size_t solver_pack_bytes(const cpphf_kernel* K);
 int solver_pack(const cpphf_kernel* K, cpphf_kernel* out, void* ws, cudaStream_t st);
 // build_fock workspace bytes for K once its packed fields exist.
 size_t fock_bytes_packed_kernel(const cpphf_kernel* K);
+// The build that fuses the assembly into the last pass for K: 1 packed, 2 many bands, 0 none.
+inline int fused_build(const cpphf_kernel* K) { return packed_fock_eligible(K) ? 1 : fock_mesh_eligible(K) ? 2 : 0; }
 // The Sigma a solver passes to build_fock: none when a build that fuses the assembly runs.
-inline double2* solver_sigma(const cpphf_kernel* K, double2* Sig) {
-    return packed_fock_eligible(K) || fock_mesh_eligible(K) ? nullptr : Sig;
-}
+inline double2* solver_sigma(const cpphf_kernel* K, double2* Sig) { return fused_build(K) ? nullptr : Sig; }
 
 }  // namespace cpphf

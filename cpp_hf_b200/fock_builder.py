@@ -21,8 +21,8 @@ later synchronisation) returns.
 
 Each ``build`` is one call of ``cpphf_build_fock`` on the current stream:
 three exchange passes and the assembly kernel (which also reduces the energy),
-or, on the Hermitian-packed path, three passes with the assembly and energy
-fused into the last.
+or, on the Hermitian-packed path and for many bands with a scalar V, three passes
+with the assembly and energy fused into the last.
 """
 
 from __future__ import annotations
@@ -41,13 +41,18 @@ class FockBuilder:
     Hermitian: when V(q) is Hermitian too (real symmetric layer-resolved V,
     real scalar V) the build then transforms the nb(nb+1)/2 upper-triangle
     channels only, with the assembly fused into the last FFT pass
-    (``packed`` tells whether that path is on)."""
+    (``packed`` tells whether that path is on: it needs mesh sides of a
+    supported length too).  ``fused`` tells whether this build writes the
+    exchange field only where it is asked for."""
 
     def __init__(self, kernel_args: dict, precision: int = 64, hermitian_density: bool = False):
         self.lib = _lib.load()
         self.dk = _DeviceKernel(kernel_args, precision=precision)
         self.dk.K.exchange_precision = int(precision)
-        self.packed = bool(hermitian_density) and self.dk.enable_packing()
+        packing = bool(hermitian_density) and self.dk.enable_packing()
+        kind = self.lib.cpphf_build_fock_fused(C.byref(self.dk.K))
+        self.fused = kind != 0
+        self.packed = packing and kind == 1
         nk1, nk2, nb = self.dk.shape
         self.shape = (nk1, nk2, nb, nb)
         dev = torch.device("cuda", torch.cuda.current_device())
@@ -83,15 +88,15 @@ class FockBuilder:
         return self.Sigma, self.F, self.E
 
     def build_fe(self, P: torch.Tensor):
-        """Fock build as the solvers run it: F and E only.  On the packed path the
-        exchange field is then never written out (the full path still needs it as
-        the assembly's input)."""
+        """Fock build as the solvers run it: F and E only.  A fused build then never
+        writes the exchange field out (the others need it as the assembly's input
+        and leave it in ``Sigma``)."""
         self._check_density(P)
         self._build_into(P, self.F, self.E)
         return self.F, self.E
 
     def _build_into(self, P: torch.Tensor, F: torch.Tensor, E: torch.Tensor):
-        sig = None if self.packed else _ptr(self.Sigma)
+        sig = None if self.fused else _ptr(self.Sigma)
         check(self.lib.cpphf_build_fock(C.byref(self.dk.K), _ptr(P), sig, _ptr(F), _ptr(self.hd),
                                         _ptr(E), None, _ptr(self.ws), self.ws.numel(), _stream()), "build_fock")
 

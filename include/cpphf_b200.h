@@ -200,9 +200,9 @@ typedef struct cpphf_kernel {
  * terms and mesh axes of a supported length; other kernels ignore the flag.
  * VR_packed / h_packed (cpphf_kernel_packed_bytes each) are made once per
  * kernel by cpphf_kernel_pack; when NULL, each build packs them into its
- * workspace (the solvers pack them once per solve).  With the flag set,
- * cpphf_build_fock accepts Sigma == NULL (no Sigma written).  No counterpart in
- * the reference for orbital V. */
+ * workspace (the solvers pack them once per solve).  Where it applies,
+ * cpphf_build_fock accepts Sigma == NULL (cpphf_build_fock_fused).  No counterpart
+ * in the reference for orbital V. */
 size_t cpphf_kernel_packed_bytes(const cpphf_kernel* K);
 /* out[0] = max |VR| and out[1] = max |VR_ba(R) - conj VR_ab(-R)| (two device
  * doubles) of a complex128 (nk1, nk2, dv, dv) VR: V(q) is Hermitian at every q
@@ -217,9 +217,12 @@ int cpphf_kernel_pack(const cpphf_kernel* K, void* VR_packed, void* h_packed, vo
  * k-independent Hartree diagonal hartree_diag (nb) and the energy
  * E = sum_k w_k Re Tr[h P + (Sigma + H)(P - refP)/2] (device scalar *energy).
  * H_dense (complex128 field, may be NULL) receives the dense Hartree term.
- * Sigma may be NULL when K's Hermitian packing applies (see cpphf_kernel) or the
- * build of many bands with a scalar V fuses the assembly; solvers then skip it.
+ * Sigma may be NULL, and is then not written, where the last pass of the exchange
+ * assembles F; solvers then skip it.  cpphf_build_fock_fused tells for K: 1 when its
+ * Hermitian packing applies (see cpphf_kernel), 2 for the build of many bands with
+ * a scalar V, 0 when Sigma is the assembly's input and must be given.
  * ---------------------------------------------------------------------- */
+int cpphf_build_fock_fused(const cpphf_kernel* K);
 size_t cpphf_build_fock_workspace_bytes(const cpphf_kernel* K);
 int cpphf_build_fock(const cpphf_kernel* K, const void* P, void* Sigma, void* F,
                      double* hartree_diag, double* energy, void* H_dense, void* workspace,
