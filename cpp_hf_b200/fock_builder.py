@@ -66,10 +66,10 @@ class FockBuilder:
     @property
     def launches_per_build(self) -> int:
         K = self.dk.K
-        pre = 2 if (K.include_hartree or K.has_contact) else 0
-        if self.packed:
+        pre = 1 if (K.include_hartree or K.has_contact) else 0  # density sum, Hartree diagonal and contact terms
+        if self.fused:
             return pre + 3  # rows forward, columns, rows inverse with the assembly and energy
-        n = 1  # bulk assembly with the energy
+        n = 1 if K.nb <= 32 else 2  # bulk assembly with the energy; above 32 bands the energy's sum on its own
         if K.include_exchange:
             n += 3
         return n + pre

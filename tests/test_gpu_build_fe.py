@@ -55,3 +55,29 @@ def test_build_fe(oracle, shape, dv, extras, kind):
     ref = oracle.build_fock_apply(args, P, None)
     assert np.abs(F1.cpu().numpy() - ref[2]).max() <= 1e-12 * max(1.0, np.abs(ref[2]).max())
     assert abs(float(E1) - ref[3]) <= 1e-12 * max(1.0, abs(ref[3]))
+
+
+@pytest.mark.parametrize("shape,dv,extras,kind", CASES, ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else str(v))
+def test_launches_per_build(native, shape, dv, extras, kind):
+    import torch
+    from cuda.bindings import runtime as rt
+
+    from cpp_hf_b200.fock_builder import FockBuilder
+
+    n1, n2, nb = shape
+    one = np.broadcast_to(np.eye(nb, dtype=complex), (n1, n2, nb, nb)).copy()
+    kw = dict(include_hartree=True, hartree_matrix=np.ones((nb, nb))) if extras else {}
+    args = problem.kernel_args(np.full((n1, n2), 1.0 / (n1 * n2)), one, np.ones((n1, n2, dv, dv)), 0.1,
+                               reference_density=0 * one, **kw)
+    fb = FockBuilder(args, hermitian_density=True)
+    P = torch.from_numpy(one).cuda()
+    fb.build_fe(P)
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        fb.build_fe(P)
+    raw = rt.cudaGraph_t(graph.raw_cuda_graph())
+    err, _, count = rt.cudaGraphGetNodes(raw)
+    assert err == rt.cudaError_t.cudaSuccess
+    err, nodes, _ = rt.cudaGraphGetNodes(raw, count)
+    kinds = [rt.cudaGraphNodeGetType(x)[1] for x in nodes]
+    assert kinds.count(rt.cudaGraphNodeType.cudaGraphNodeTypeKernel) == fb.launches_per_build
