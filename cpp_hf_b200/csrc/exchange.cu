@@ -970,6 +970,10 @@ int exchange_hcp_two_passes(const double2* P, const double2* refP, const double2
 bool hcp_tiled(int64_t n0, int64_t n1, int64_t nb) {
     if (nb <= 8 || nb > 4096 || n0 > 65535 || n1 > 65535 || split_of((int)n1).n1 == 0) return false;
     const int64_t tiled = hcp_channels(2, (int)nb), tri = hcp_channels(1, (int)nb), field = n0 * n1 * nb * nb;
+    // the passes put chunks of 16 channels, of 8 on lines of more than 16 lanes, along grid.y
+    const Split a = split_of((int)n0), b = split_of((int)n1);
+    const int64_t chunk = std::max({a.n1, a.n2, b.n1, b.n2}) <= 16 ? 16 : 8;
+    if (tiled / chunk > 65535) return false;
     return field >= (int64_t)1 << 22 && (10 * tiled <= 13 * tri || (10 * tiled <= 16 * tri && field >= (int64_t)1 << 23));
 }
 
