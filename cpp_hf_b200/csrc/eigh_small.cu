@@ -44,7 +44,7 @@ constexpr int kGroup = 8;  // lanes per matrix of the group form
 constexpr double kTinyNorm2 = 1e-290;
 __device__ __forceinline__ double modulus(double2 x) {
     const double m2 = fma(x.x, x.x, x.y * x.y);
-    return m2 > kTinyNorm2 ? sqrt(m2) : 0.0;
+    return m2 <= kTinyNorm2 ? 0.0 : sqrt(m2);  // a NaN stays one
 }
 
 template <int GS>
@@ -115,10 +115,10 @@ __global__ void __launch_bounds__(kHqlThreads, 4) k_eigh_hql(const double2* __re
             for (int i = kk + 1; i < NB; ++i) xn2 += a[i].x * a[i].x + a[i].y * a[i].y;
             const double2 x0 = a[kk + 1];
             const double ax0 = modulus(x0);
-            const double xn = xn2 > kTinyNorm2 ? sqrt(xn2) : 0.0;
+            const double xn = xn2 <= kTinyNorm2 ? 0.0 : sqrt(xn2);
 #pragma unroll
             for (int i = 0; i < NB; ++i) ul[i] = mk(0.0, 0.0);
-            if (xn > 0.0) {
+            if (!(xn <= 0.0)) {  // or NaN
                 const double iax = ax0 > 0.0 ? 1.0 / ax0 : 0.0;
                 const double2 ph = ax0 > 0.0 ? mk(x0.x * iax, x0.y * iax) : mk(1.0, 0.0);
                 al = mk(-ph.x * xn, -ph.y * xn);
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(kThreadCta, 4)
             for (int i = kk + 1; i < NB; ++i) xn2 += a[i][kk].x * a[i][kk].x + a[i][kk].y * a[i][kk].y;
             const double2 x0 = a[kk + 1][kk];
             const double ax0 = modulus(x0), xn = sqrt(xn2);
-            const bool on = xn2 > kTinyNorm2;
+            const bool on = !(xn2 <= kTinyNorm2);  // or NaN
             const double iax = ax0 > 0.0 ? 1.0 / ax0 : 0.0;
             const double2 ph = ax0 > 0.0 ? mk(x0.x * iax, x0.y * iax) : mk(1.0, 0.0);
             // beta = 1 / (xn (xn + ax0)); u is scaled by its square root
