@@ -83,7 +83,8 @@ __global__ void k_pack_fields(const double2* __restrict__ VR, int dv, const doub
 // mod n on both axes), as the bit patterns of non-negative doubles, whose integer
 // order is theirs (a NaN is above all).
 __device__ __forceinline__ unsigned long long bits_abs(double2 v) {
-    return (unsigned long long)__double_as_longlong(hypot(v.x, v.y)) & 0x7fffffffffffffffull;
+    const double m = isnan(v.x) || isnan(v.y) ? NAN : hypot(v.x, v.y);  // hypot(NaN, inf) is inf
+    return (unsigned long long)__double_as_longlong(m) & 0x7fffffffffffffffull;
 }
 __global__ void k_vr_hermitian(const double2* __restrict__ VR, int n0, int n1, int dv, unsigned long long* out) {
     const int dv2 = dv * dv;
