@@ -62,18 +62,24 @@ __global__ void __launch_bounds__(kRhoThreads)
     const bool live = lane < lanes && c < nb2;
     const int64_t per = (nk + Gk - 1) / Gk, k0 = blockIdx.x * per, k1 = min(nk, k0 + per);
     double2 acc = mk(0.0, 0.0);
-    // acc of lane 0 <- the channel's sum over the lanes: a tree, since one or two bands
-    // leave 1024 or 256 lanes to a channel (one band at 192 x 192, whole build: 46 us, with
-    // the lanes added one by one 68)
+    // acc of lane 0 <- the channel's sum over the lanes, one by one; in two steps of their
+    // square root for the 1024 lanes of a single band (192 x 192, whole build: 44 us, one
+    // by one 68).  At 256 lanes (two bands) the steps gain 3 us, at 113 and below nothing
+    // (75 x 98, nb = 5: a barrier per level of a tree took 62.2 against 61.6).
     auto lane_sum = [&]() {
         acc_sh[tid] = acc;
-        for (int s = 1 << (31 - __clz(lanes - 1)); s > 0; s >>= 1) {
-            __syncthreads();
-            if (live && lane < s && lane + s < lanes) {
-                acc = cadd(acc, acc_sh[(lane + s) * CH + cl]);
+        __syncthreads();
+        int n = lanes;
+        if (lanes > 256) {
+            n = 1 << ((33 - __clz(lanes - 1)) / 2);
+            if (live && lane < n) {
+                for (int l = lane + n; l < lanes; l += n) acc = cadd(acc, acc_sh[l * CH + cl]);
                 acc_sh[tid] = acc;
             }
+            __syncthreads();
         }
+        if (lane == 0 && live)
+            for (int l = 1; l < n; ++l) acc = cadd(acc, acc_sh[l * CH + cl]);
     };
     if (live) {
         int64_t k = k0 + lane;
