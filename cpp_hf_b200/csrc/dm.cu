@@ -275,7 +275,8 @@ void init_attrs() {
 
 int dm_check_nb(int64_t nb) {
     if (nb < 1) return fail(CPPHF_ERR_INVALID, "nb must be positive");
-    // three team matrices of nb x (nb + 1) complex128 must fit in 227 KB (nb <= 68)
+    // nb <= 68: three team matrices of nb x (nb + 1) complex128 in 227 KB, as the spectral
+    // diagonal (k_diag_ufu) holds them; the solvers' tensor-core kernels go to 72
     if (sizeof(double2) * team_mat_elems((int)nb) * 3 + 64 * sizeof(double) + 4 * nb * sizeof(double2) > 227 * 1024)
         return fail(CPPHF_ERR_UNSUPPORTED, "nb too large for the per-k shared-memory kernels");
     return CPPHF_OK;

@@ -1,5 +1,6 @@
 // Batched Hermitian eigendecomposition for any nb <= kMaxEighNb (replaces
-// Eigen's SelfAdjointEigenSolver in cpp_hf linalg.hpp:39-120): Householder
+// Eigen's SelfAdjointEigenSolver in cpp_hf linalg.hpp:39-120; nb <= 8 and block
+// structures of small blocks run eigh_small.cu): Householder
 // reduction to a real symmetric tridiagonal, divide and conquer on it, and the
 // back-transformation, one CTA per matrix in one launch.
 //
@@ -9,7 +10,7 @@
 // p broadcast from shared memory.
 //  1. Reduction, k = 0 .. n-3: H = I - beta u u^H maps A[k+1:, k] to alpha e1;
 //     with p = beta A u, K = beta/2 u^H p and w = p - K u the similarity is the
-//     rank-2 update A -= u w^H + w u^H.  Two block barriers a step.  A unitary
+//     rank-2 update A -= u w^H + w u^H.  Three block barriers a step.  A unitary
 //     diagonal makes the subdiagonal e real and non-negative.
 //  2. Divide and conquer (Cuppen 1981; Gu and Eisenstat 1995): T is torn at
 //     every off-diagonal, T = diag(d_i - e_{i-1} - e_i) + sum e_i v_i v_i^T, and
@@ -20,7 +21,9 @@
 //     iteration (Li 1993) inside a bisection bracket; z is recomputed from the
 //     roots (Loewner's formula), which makes the eigenvectors orthogonal to
 //     rounding; the vectors are the product of the old ones with
-//     z_i / (d_i - x).  No step is a chain longer than one row of the matrix,
+//     z_i / (d_i - x).  The deflation tolerance, the choice of the root formula in the
+//     iteration and its fallback are those of LAPACK's dlaed2 and dlaed4 (LAPACK
+//     Working Notes 69 and 89).  No step is a chain longer than one row of the matrix,
 //     unlike the n^2 dependent rotations of QL.
 //  3. The reflectors are applied to the eigenvectors, stored by ascending
 //     eigenvalue (stable) or, with block sizes, block by block.

@@ -3,7 +3,7 @@
 // iterations, everything in registers (replaces Eigen's SelfAdjointEigenSolver in
 // cpp_hf linalg.hpp:39-66, which takes the same tridiagonal + QL route): eight
 // lanes per matrix for small batches of nb = 5..8, one thread per matrix
-// otherwise (k_eigh_thread, below).
+// otherwise, also for the blocks of block-diagonal matrices (k_eigh_thread, below).
 //
 // Lane r of a group owns column r of A and row r of the accumulated unitary Z.
 //  1. Reduction, k = 0 .. nb-3: lane k forms the reflector H = I - beta u u^H
@@ -15,11 +15,11 @@
 //     is a row-local update.
 //  2. A unitary diagonal D (delta_0 = 1, delta_{k+1} = delta_k e_k/|e_k|) makes
 //     the tridiagonal real: T' = D^H T D, Z <- Z D.
-//  3. Implicit QL with Wilkinson shifts on (d, |e|) (Golub & Van Loan,
-//     Matrix Computations, sec. 8.3; the tqli formulation of Press et al.):
-//     every lane runs the same scalar recurrence and applies each Givens
-//     rotation to its own row of Z.  The matrix is first scaled by a power of
-//     two (exact) so that each rotation can use one reciprocal square root.
+//  3. Implicit QL with Wilkinson shifts on (d, |e|) (the recurrence of EISPACK's
+//     imtql2; Golub & Van Loan, Matrix Computations, sec. 8.3): every lane runs
+//     the same scalar recurrence and applies each Givens rotation to its own row
+//     of Z.  The matrix is first scaled by a power of two (exact) so that each
+//     rotation can use one reciprocal square root.
 //  4. Stable ascending sort of the eigenvalues, columns of Z permuted to match.
 // Loops over matrix indices are unrolled with compile-time indices so the
 // per-lane arrays stay in registers.

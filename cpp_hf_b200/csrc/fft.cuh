@@ -1,5 +1,6 @@
-// Generic shared-memory batched 1-D FFT (the complex64 exchange) on a tile of n points x CB channels,
-// for line lengths that have no register codelet (fft_reg.cuh).
+// Generic shared-memory batched 1-D FFT on a tile of n points x CB channels, for line
+// lengths that have no register codelet (fft_reg.cuh): the complex64 exchange, and the
+// complex128 passes too small for the mixed-radix ones (exchange_smooth.cu).
 //
 // The tile is row-major [n][CB] complex in shared memory (channel fastest).  A
 // plan is a list of radices whose product is n; every stage is an out-of-place

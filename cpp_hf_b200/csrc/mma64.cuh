@@ -19,8 +19,6 @@
 
 namespace cpphf {
 
-constexpr int kMmaMaxTiles = 9;  // nb <= 72
-
 template <int NT>
 struct MmaGeo {
     static constexpr int NP = 8 * NT, LD = NP + 1;
@@ -32,9 +30,6 @@ struct MmaGeo {
     static constexpr int BLOCKS = NT <= 2 ? 3 : NT == 3 ? 4 : NT == 4 ? 5 : NT == 5 ? 4 : NT == 6 ? 3 : NT <= 8 ? 2 : 1;
     static constexpr size_t MAT = (size_t)NP * LD;  // complex elements of one matrix in shared memory
 };
-
-template <int NT>
-using MmaAcc = double2[NT][2];
 
 // barrier of the calling thread's group
 template <int NT>

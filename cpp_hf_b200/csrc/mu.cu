@@ -19,9 +19,10 @@
 // its sums into its slot and every block polls all slots until they hold numbers.
 // The sums are their own flags, so a round is one store and one L2 round trip
 // instead of a counter, a generation word, their fences and a second read.
-// Measured against that barrier (bisection / in-loop Newton, us): 294912
-// eigenvalues 78 / 57 -> 60 / 35, 82944 66 / 55 -> 54 / 40, 4608 103 / 57 -> 27 / 16.5
-// (one block -> one cluster).
+// Measured against that barrier (bisection / in-loop Newton, us, means of 12
+// problems): 1327104 eigenvalues 159 / 98 -> 145 / 91, 294912 82 / 50 -> 68 / 41, 65536
+// 143 / 74 -> 106 / 63 (one cluster, its sums in distributed shared memory now), 4608
+// 104 / 70 -> 25 / 17 (one block -> one cluster).
 #include "common.cuh"
 #include "mu.cuh"
 

@@ -459,10 +459,10 @@ struct SolveStream {
 };
 
 // Iterations launched kernel by kernel before one is captured.  A capture costs
-// about 340 us for the two parities of a DM iteration and 180 us for an SCF
-// iteration, and saves 25 to 35 us on each iteration after it, so a solve that is
-// done by then is better off without (measured on 48 x 48, nb = 2, and on
-// 192 x 192, nb = 8).
+// about 390 us for the two parities of a DM iteration and 100 to 180 us for an SCF
+// iteration, and saves 20 to 28 us on each iteration after it, so a solve that is
+// done by then is better off without.  Measured on 192 x 192, nb = 8, with graphs less
+// without, us: DM 14 iterations +389, 24 +80, 34 -202; SCF 10 +73, 20 -164, 30 -405.
 constexpr int64_t kGraphAfterDm = 12;
 constexpr int64_t kGraphAfterScf = 8;
 
