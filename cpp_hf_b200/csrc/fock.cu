@@ -47,6 +47,8 @@ constexpr int kTileElems = 1024;  // k-blocks of at most this many elements take
 constexpr int kRhoThreads = 1024;
 constexpr int kRhoChannels = 256;
 
+// TWO_STEP: more than 256 lanes to a channel (a single band).
+template <bool TWO_STEP>
 __global__ void __launch_bounds__(kRhoThreads)
     k_hartree_contact(const double2* __restrict__ P, const double2* __restrict__ refP, const double* __restrict__ w,
                       int64_t nk, int nb, int CH, double2* part, unsigned* counter, const double* __restrict__ HH,
@@ -70,7 +72,7 @@ __global__ void __launch_bounds__(kRhoThreads)
         acc_sh[tid] = acc;
         __syncthreads();
         int n = lanes;
-        if (lanes > 256) {
+        if constexpr (TWO_STEP) {
             n = 1 << ((33 - __clz(lanes - 1)) / 2);
             if (live && lane < n) {
                 for (int l = lane + n; l < lanes; l += n) acc = cadd(acc, acc_sh[l * CH + cl]);
@@ -469,7 +471,8 @@ int build_fock(const cpphf_kernel* K, const double2* P, double2* Sigma, double2*
         unsigned* rho_counter = reinterpret_cast<unsigned*>(W + L.off_rho_counter);
         CPPHF_CUDA(cudaMemsetAsync(rho_counter, 0, sizeof(unsigned) * (1 + (size_t)L.slices), st));
         // the superlattice Hartree replaces the diagonal Hartree (fock.hpp:66-175)
-        k_hartree_contact<<<dim3(L.Gk, L.slices), kRhoThreads, 0, st>>>(
+        auto kern = kRhoThreads / L.CH > 256 ? k_hartree_contact<true> : k_hartree_contact<false>;
+        kern<<<dim3(L.Gk, L.slices), kRhoThreads, 0, st>>>(
             P, refP, K->w2d, nk, nb, L.CH, rho_part, rho_counter, K->HH, K->include_hartree && !slh, K->has_contact,
             K->n_contact, K->contact_g, static_cast<const double2*>(K->contact_Oi),
             static_cast<const double2*>(K->contact_Oj), rho_bar, hd, SC);
